@@ -12,7 +12,9 @@
 //     fractional remainder), and the profile is evaluated with the SFU
 //     (lg2/ex2) -- together with its analytic derivatives for the gradient.
 #pragma once
+#include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <cuda_runtime.h>
 
 #ifndef __CUDACC__
@@ -75,6 +77,11 @@ struct CompF64 {
   double cosPA, sinPA, q;
   double a, b, c, d, e, f;      // type-specific (see comp_setup64)
   double g, h, i, j, k, l, m;   // 3-D functions
+  // the radial classes' few-instruction form (comp_fast64): 1/q and the
+  // type's constants, as unevaluated sums, and the high word of
+  // X^2 + (Y/q)^2 from which it is used
+  double iqh, iql, u, uh, ul, vh, vl;
+  int farHi, pad2;
 };
 
 // FP32 fast-path state prepared once per parameter vector.
@@ -230,6 +237,75 @@ __host__ __device__ inline int n_subsamples64(const CompF64 &c, double r) {
     ns = (k < 100) ? k : 100;
   }
   return ns;
+}
+
+// Constants of the few-instruction form of a radial class (host), as
+// unevaluated sums h + l of two doubles:
+//   iqh + iql = 1/q
+//   Sersic:   u = 1/(2n); uh + ul = b_n log2 e; vh + vl = 2 log2 r_e, vh a multiple of 2^-40
+//   Exp:      uh + ul = log2 e / h
+//   GRing, Gaussian: uh + ul = log2 e / (2 sigma^2)
+//   Moffat:   u = -beta; uh + ul = 1/alpha^2
+// The low parts cost four to six instructions a pixel and keep the constants'
+// rounding out of the image, as the reference's divisions do.
+// farHi: above it the form is used.  Nearer than radius 10 a pixel of a
+// subsampling class may be subsampled, and the count (int)(20/r) must see the
+// radius as the reference rounds it, so those pixels keep the reference's
+// expressions (1 % margin; unsubsampled classes only the innermost 1e-4
+// pixels); INT_MAX keeps every pixel on them, for parameters outside the
+// form's range (a non-positive scale or axis ratio).
+inline void hl_quotient(double num, double numLow, double den, double &h, double &l) {
+  h = num / den;
+  l = (fma(-h, den, num) + numLow) / den;
+}
+inline void comp_fast64(CompF64 &c, bool enable) {
+  c.iqh = c.iql = c.u = c.uh = c.ul = c.vh = c.vl = 0.0;
+  c.farHi = 0x7fffffff;
+  if (!enable) return;
+  // log2 e to 107 bits
+  const double e2h = 1.4426950408889634, e2l = 2.0355273740931033e-17;
+  double scale;
+  switch (c.type) {
+    case F_SERSIC: scale = c.c; break;
+    case F_EXP: scale = c.b; break;
+    case F_MOFFAT: scale = c.d; break;
+    case F_GRING: scale = c.c; break;
+    case F_GAUSS: scale = c.b; break;
+    default: return;
+  }
+  if (!(scale > 1e-6 && scale < 1e12 && c.q > 1e-6 && c.q < 1e6)) return;
+  if (c.type == F_SERSIC && !(c.a > 0.02 && c.a < 1e3 && c.d == c.d)) return;
+  if (c.type == F_MOFFAT && !(c.c > -1e3 && c.c < 1e3)) return;
+  if (!(c.x0 > -1e9 && c.x0 < 1e9 && c.y0 > -1e9 && c.y0 < 1e9)) return;
+  hl_quotient(1.0, 0.0, c.q, c.iqh, c.iql);
+  switch (c.type) {
+    case F_SERSIC: {
+      c.u = 0.5 * c.e;
+      c.uh = c.d * e2h;
+      c.ul = fma(c.d, e2h, -c.uh) + c.d * e2l;
+      // (long double: 64 bits on x86, 113 on Arm)
+      const long double x = 2.0L * log2l((long double)c.c);
+      c.vh = nearbyint((double)x * 1099511627776.0) / 1099511627776.0;
+      c.vl = (double)(x - (long double)c.vh);
+      break;
+    }
+    case F_EXP: hl_quotient(e2h, e2l, c.b, c.uh, c.ul); break;
+    case F_GRING: case F_GAUSS: hl_quotient(e2h, e2l, c.d, c.uh, c.ul); break;
+    case F_MOFFAT: {
+      c.u = -c.c;
+      const double a2 = c.d * c.d, low = fma(c.d, c.d, -a2);
+      hl_quotient(1.0, 0.0, a2, c.uh, c.ul);
+      c.ul -= c.uh * (low / a2);
+      break;
+    }
+    default: break;
+  }
+  const bool sub = c.subsample && c.type != F_GRING;
+  const double rmin = sub ? 10.1 : 1e-4;
+  const double v = rmin * rmin;
+  unsigned long long bits;
+  memcpy(&bits, &v, sizeof bits);
+  c.farHi = (int)(bits >> 32) + 1;
 }
 
 // CalculateIntensity(r) of the radial classes, FP64.

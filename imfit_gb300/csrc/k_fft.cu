@@ -13,6 +13,8 @@
 //   3. k_rows_c2r   : each needed row -> real row, rescaled.
 // Padded lengths are 7-smooth, at least as large as the reference's
 // (N + P - 1); linear convolution is unchanged by extra zero padding.
+#include <algorithm>
+
 #include "kernels.h"
 #include "fft.cuh"
 
@@ -159,14 +161,28 @@ static const cplx<T> *twl_of(const FFTLen &L) {
   return reinterpret_cast<const cplx<T> *>(sizeof(T) == 8 ? (const void *)L.twL64 : (const void *)L.twL32);
 }
 
-// One line per CTA and about one thread per complex point: the FFT passes of a
-// line then have one butterfly per thread, and many small CTAs keep the SMs
-// occupied even for a single image.
+// One line per CTA (many small CTAs keep the SMs occupied even for a single
+// image).
 int rows_per_block(int M, int elemBytes, int nbuf) {
   (void)M;
   (void)elemBytes;
   (void)nbuf;
   return 1;
+}
+
+// Threads of a CTA that transforms one line of n FP64 complex points.  The
+// FP64 pipe is full with a few warps per SM, and what counts beside it is that
+// the lines' memory phases overlap other lines' arithmetic: few threads, so
+// that about five CTAs share an SM (a 1250-point column pass of 626 columns
+// then is one wave instead of two).  Launches of fewer than four lines per SM
+// take one thread per four points instead: their time is the latency of one line.
+static int fp64_line_threads(int n, long lines) {
+  if (lines < 4 * 152) return std::max(64, std::min(1024, (n / 4 + 31) / 32 * 32));
+  return n < 640 ? 64 : (n < 2048 ? 128 : 256);
+}
+template <typename T>
+static int row_threads(int M, long lines) {
+  return sizeof(T) == 8 ? fp64_line_threads(M, lines) : line_threads(M);
 }
 
 int line_threads(int points) {
@@ -185,14 +201,15 @@ cudaError_t launch_rows_r2c(const T *in, long inPitch, long inBatch, int inCols,
   auto kern = k_rows_r2c<T>;
   allow_max_smem((const void *)kern);
   dim3 grid((nRows + rpb - 1) / rpb, nBatch);
-  kern<<<grid, line_threads(M * rpb), sm, st>>>(in, inPitch, inBatch, inCols, nRows, reinterpret_cast<cplx<T> *>(out), outPitch,
+  kern<<<grid, row_threads<T>(M, (long)nRows * nBatch), sm, st>>>(in, inPitch, inBatch, inCols, nRows, reinterpret_cast<cplx<T> *>(out), outPitch,
                               outBatch, plan_of<T>(Lx, true), twl_of<T>(Lx), rpb);
   return cudaGetLastError();
 }
 
 int cols_per_block(int Ly, int elemBytes, int nColsC) {
-  // two ping-pong buffers of Ly x cpb complex per CTA; one or two columns per
-  // CTA, two only when that still leaves several CTAs per SM
+  // two ping-pong buffers of Ly x cpb complex per CTA; FP64: one column (see
+  // fp64_line_threads); FP32: two only when that still leaves several CTAs per SM
+  if (elemBytes == 8) return 1;
   int cpb = (nColsC >= 600) ? 2 : 1;
   while (cpb > 1 && (size_t)2 * Ly * cpb * 2 * elemBytes > 200 * 1024) cpb >>= 1;
   return cpb;
@@ -208,7 +225,9 @@ cudaError_t launch_cols(void *spec, long pitch, long batch, int nColsC, int nRow
   while (cpb > 1 && (size_t)2 * L * cpb * 2 * sizeof(T) > 200 * 1024) cpb >>= 1;
   const size_t sm = sizeof(cplx<T>) * 2 * (size_t)L * cpb;
   dim3 grid((nColsC + cpb - 1) / cpb, nBatch);
-  const int nt = threadsOverride > 0 ? threadsOverride : line_threads(L * cpb / 2);
+  const int nt = threadsOverride > 0 ? threadsOverride
+                 : sizeof(T) == 8    ? fp64_line_threads(L, (long)nColsC * nBatch)
+                                     : line_threads(L * cpb / 2);
   auto p = plan_of<T>(Ly, false);
   cplx<T> *s = reinterpret_cast<cplx<T> *>(spec);
   const cplx<T> *h = reinterpret_cast<const cplx<T> *>(H);
@@ -235,7 +254,7 @@ cudaError_t launch_rows_c2r(const void *in, long inPitch, long inBatch, int nRow
   auto kern = k_rows_c2r<T>;
   allow_max_smem((const void *)kern);
   dim3 grid((nRows + rpb - 1) / rpb, nBatch);
-  kern<<<grid, line_threads(M * rpb), sm, st>>>(reinterpret_cast<const cplx<T> *>(in), inPitch, inBatch, nRows, out, outPitch,
+  kern<<<grid, row_threads<T>(M, (long)nRows * nBatch), sm, st>>>(reinterpret_cast<const cplx<T> *>(in), inPitch, inBatch, nRows, out, outPitch,
                               outBatch, outCols, scale, plan_of<T>(Lx, true), twl_of<T>(Lx), rpb);
   return cudaGetLastError();
 }

@@ -135,15 +135,20 @@ struct Grid64 {
   int isRegion;
   int x1, y1;
   double off, frac;
-  // subsampled pixels, computed beforehand by one warp each: sub[c][S*S] over
-  // a box of S = 2 subHalf pixels around component c's centre (null: each
-  // pixel's thread sums its subsamples itself)
+  // subsampled pixels, computed beforehand: sub[vector][c][S*S] over a box of
+  // S = 2 subHalf pixels around component c's centre
   double *sub;
   int subHalf;
+  // region: its scale, and the shared subsample lattice's scratch (null:
+  // every pixel sums its own subsamples)
+  int scale;
+  double *lattice;
 };
 
-// Scratch size (doubles) of the subsampled-pixel table of nComp components on g.
+// Scratch sizes (doubles) of nComp components on g: the subsampled-pixel
+// table and the lattice (0: the grid has none).
 size_t sub_table_size(const Grid64 &g, int nComp);
+size_t lattice_size(const Grid64 &g, int nComp);
 
 // 3-D (line-of-sight) components of a model: their indices in the component
 // list; component c's CompF64::pad0 holds its position k3 in this list.
@@ -160,7 +165,8 @@ cudaError_t launch_flux64(const CompF64 &c, int xSize, int ySize, double *partia
                           cudaStream_t st);
 // model pixels; 3-D components are read from 'los' (may be null without them)
 cudaError_t launch_eval64(const CompF64 *comps, int nComp, double *model, long pitch, Grid64 g,
-                          const double *los, cudaStream_t st);
+                          const double *los, cudaStream_t st, int nVec = 1, long modelStride = 0,
+                          double *base = nullptr, const unsigned *changed = nullptr);
 // point sources the fast path evaluates (per model)
 constexpr int kMaxPsFast = 8;
 
@@ -171,9 +177,9 @@ struct PsScales {
 // point sources after the convolution
 cudaError_t launch_point_sources64(const CompF64 *comps, int nComp, double *model, long pitch, Grid64 g,
                                    PsfInterp<double> ip, const PsScales &scales, cudaStream_t st);
-cudaError_t launch_downsample64(const double *region, int nOC, int nOR, int osPsfCols, int osPsfRows,
-                                double *mainImg, int nMainCols, int nMainRows, int mainPsfCols,
-                                int mainPsfRows, int x1, int y1, int scale, cudaStream_t st);
+cudaError_t launch_downsample64(const double *region, int nOC, int padC, int padR, int nColsSub, int nRowsSub,
+                                double *mainImg, int nMainCols, int mainPsfCols, int mainPsfRows, int x1, int y1,
+                                int scale, cudaStream_t st, int nVec = 1, long regionStride = 0, long mainStride = 0);
 
 // statistic over the data crop (FP64).  kind: 0 chi^2 (enorm^2), 1 Cash, 2 PMLR-Cash
 struct StatArgs64 {
@@ -193,9 +199,13 @@ struct StatArgs64 {
 cudaError_t launch_deviates64(const StatArgs64 &a, double *dev, double *wOut, cudaStream_t st);
 // deterministic two-level reduction; partials must hold >= kStatBlocks * 8 doubles
 constexpr int kStatBlocks = 296;
-cudaError_t launch_statistic64(const StatArgs64 &a, double *partials, double *result, cudaStream_t st);
-// one finite-difference gradient column: out = sum_z dev0_z * (dev1_z - dev0_z) / h  (deterministic)
-cudaError_t launch_fd_dot64(const double *dev0, const double *dev1, long n, double invh, double *partials,
+// of nVec model images modelStride apart (that many partials and results)
+cudaError_t launch_statistic64(const StatArgs64 &a, double *partials, double *result, cudaStream_t st, int nVec = 1,
+                               long modelStride = 0);
+// nCols finite-difference columns of the chi^2 gradient: result[j] = 2 sum_z
+// dev0_z (dev_(1+j)z - dev0_z) invh[j] with the deviates of the model images
+// a.model + v modelStride (deterministic)
+cudaError_t launch_fd_dot64(const StatArgs64 &a, long modelStride, int nCols, const double *invh, double *partials,
                             double *result, cudaStream_t st);
 cudaError_t launch_crop64(const double *model, int modelCols, int offR, int offC, int nCols, int nRows,
                           double *out, cudaStream_t st);

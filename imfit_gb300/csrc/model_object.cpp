@@ -176,6 +176,22 @@ struct DevBuf {
   }
 };
 
+// A grid that a region's model is evaluated and convolved on: gridCols x
+// gridRows subpixels, the region's first one padC x padR inside it.
+struct RegionGrid {
+  bool ready = false;
+  int cols = 0, rows = 0, padC = 0, padR = 0;
+  long vals = 0;
+  FFTLen Lx, Ly;
+  DevBuf<double> model;
+  DevBuf<double> spec;  // complex, Ly x (Lx/2+1)
+  DevBuf<double> H;     // complex
+  ~RegionGrid() {
+    fftlen_destroy(Lx);
+    fftlen_destroy(Ly);
+  }
+};
+
 struct Region {
   int x1, y1, nBaseCols, nBaseRows, scale;
   int nPsfCols, nPsfRows;
@@ -184,13 +200,17 @@ struct Region {
   DevBuf<double> psTab;        // that interpolator's tables
   PsfInterp<double> ps64{};
   double psfSum = 1.0;
-  int nModelCols, nModelRows;
-  long nModelVals;
-  FFTLen Lx, Ly;
-  DevBuf<double> model;
-  DevBuf<double> spec;   // complex, Ly x (Lx/2+1)
-  DevBuf<double> H;      // complex
+  int nModelCols, nModelRows;  // the reference's region model
   int nColsSub, nRowsSub;
+  // Of the region model only the subpixels of the replaced data pixels are
+  // read back, so the "valid window" -- those and the PSF's reach around
+  // them -- is enough (40 x 40 pixels at 5x with a 315 x 315 PSF: 514^2
+  // subpixels and a 525-point FFT instead of 830^2 and 1152: 0.84 of the
+  // 1024 x 1024 benchmark model's 2.23 ms, now 0.16).  The full model where
+  // the reference's size rule reads beyond the region's own subpixels, and
+  // for finite differences (see fdGradient), which make it when first asked.
+  RegionGrid win, full;
+  bool windowed = false;
 };
 
 struct Captured {
@@ -251,10 +271,11 @@ struct imfit_model_s {
   MT19937 rng;
 
   std::vector<Region *> regions;
+  bool refArith = false;  // evaluate with the reference's expressions throughout (finite differences)
 
   // plain FP64 device state
   FFTLen Lx, Ly;
-  DevBuf<double> dModel, dSpec, dH, dData, dWeight, dMask, dExtra, dDev, dDev2, dPart, dRes;
+  DevBuf<double> dModel, dSpec, dH, dData, dWeight, dMask, dExtra, dDev, dPart, dRes;
   DevBuf<long> dBoot;
   DevBuf<CompF64> dComps;
   std::vector<CompF64> hComps;
@@ -262,6 +283,11 @@ struct imfit_model_s {
   LosList64 losList{};
   DevBuf<double> dLos;
   DevBuf<double> dSub;  // subsampled-pixel table of the plain path (k_sub64)
+  // batched finite-difference gradient: models, spectra, region models side by
+  // side, vector 0's component values, steps and changed components
+  DevBuf<double> dFdModel, dFdSpec, dFdRegion, dFdBase, dFdInvH;
+  DevBuf<unsigned> dFdChanged;
+  DevBuf<double> dLattice;  // its regions' shared subsample lattice (k_lattice64)
   DevBuf<int> dLosFlag;
   int *hLosFlag = nullptr;  // pinned copy of the "list too short" flag
   double *hPinned = nullptr;  // pinned scratch for small transfers
@@ -365,11 +391,7 @@ struct imfit_model_s {
   bool concurrent = true;
 
   ~imfit_model_s() {
-    for (Region *r : regions) {
-      fftlen_destroy(r->Lx);
-      fftlen_destroy(r->Ly);
-      delete r;
-    }
+    for (Region *r : regions) delete r;
     fftlen_destroy(Lx);
     fftlen_destroy(Ly);
     fftlen_destroy(Fx);
@@ -538,7 +560,6 @@ struct imfit_model_s {
     for (double v : r->psf) r->psfSum += v;
     r->nModelCols = r->nBaseCols * scale + 2 * pc;
     r->nModelRows = r->nBaseRows * scale + 2 * pr;
-    r->nModelVals = (long)r->nModelCols * r->nModelRows;
     r->nColsSub = (r->nModelCols - 2 * pc) / scale;
     r->nRowsSub = (r->nModelCols - 2 * pr) / scale;  // core/downsample.cpp:79 uses the column count
     // the reference reads region-model rows up to (nRowsSub)*k + pr - 1 and
@@ -551,27 +572,51 @@ struct imfit_model_s {
       return fail(IMFIT_E_UNSUPPORTED,
                   "oversampled region shape would make DownsampleAndReplace read/write outside its images");
     }
-    int e1 = fftlen_create(r->Lx, smooth_size(r->nModelCols + pc - 1, true), kRadixPlain);
-    int e2 = fftlen_create(r->Ly, smooth_size(r->nModelRows + pr - 1, true), kRadixPlain);
-    if (e1 || e2) {
-      delete r;
-      return fail(IMFIT_E_CUDA, "FFT tables");
-    }
-    int st = spectrum64(wrap_psf(r->psf, pc, pr, r->Lx.L, r->Ly.L), r->Lx, r->Ly, r->H);
-    if (st) {
+    r->windowed = r->nColsSub <= r->nBaseCols && r->nRowsSub <= r->nBaseRows;
+    if (int st = makeRegionGrid(*r, r->windowed ? r->win : r->full, r->windowed)) {
       delete r;
       return st;
-    }
-    cudaError_t e = r->model.reserve(r->nModelVals);
-    if (!e) e = r->spec.reserve(2 * (size_t)r->Ly.L * (r->Lx.L / 2 + 1));
-    if (e) {
-      delete r;
-      return cuda_fail(e, "region buffers");
     }
     regions.push_back(r);
     fastReady = false;
     return 0;
   }
+
+  // Buffers and PSF spectrum of a region's valid window or of its full model
+  // (the reference's padding; kept when already made).
+  int makeRegionGrid(Region &r, RegionGrid &g, bool window) {
+    if (g.ready) return 0;
+    const int pc = r.nPsfCols, pr = r.nPsfRows;
+    int Lx0, Ly0;
+    if (window) {
+      // a circular length of the window itself: no wrapped term reaches the
+      // subpixels that are read
+      g.cols = Lx0 = r.nColsSub * r.scale + pc - 1;
+      g.rows = Ly0 = r.nRowsSub * r.scale + pr - 1;
+      g.padC = pc - 1 - pc / 2;
+      g.padR = pr - 1 - pr / 2;
+    } else {
+      g.cols = r.nModelCols;
+      g.rows = r.nModelRows;
+      g.padC = pc;
+      g.padR = pr;
+      Lx0 = r.nModelCols + pc - 1;
+      Ly0 = r.nModelRows + pr - 1;
+    }
+    g.vals = (long)g.cols * g.rows;
+    if (fftlen_create(g.Lx, smooth_size(Lx0, true), kRadixPlain) ||
+        fftlen_create(g.Ly, smooth_size(Ly0, true), kRadixPlain))
+      return fail(IMFIT_E_CUDA, "FFT tables");
+    int st = spectrum64(wrap_psf(r.psf, pc, pr, g.Lx.L, g.Ly.L), g.Lx, g.Ly, g.H);
+    if (st) return st;
+    cudaError_t e = g.model.reserve(g.vals);
+    if (!e) e = g.spec.reserve(2 * (size_t)g.Ly.L * (g.Lx.L / 2 + 1));
+    if (e) return cuda_fail(e, "region buffers");
+    g.ready = true;
+    return 0;
+  }
+  // the grid an evaluation uses
+  RegionGrid &gridOf(Region &r) const { return r.windowed && !refArith ? r.win : r.full; }
 
   // GenerateErrorVector (core/model_object.cpp:642-673)
   void generateErrorVector() {
@@ -646,7 +691,6 @@ struct imfit_model_s {
     if (!e) e = dMask.reserve(n);
     if (!e) e = dExtra.reserve(n);
     if (!e) e = dDev.reserve(n);
-    if (!e) e = dDev2.reserve(n);
     if (!e) e = dPart.reserve(kStatBlocks * 8);
     if (!e) e = dRes.reserve(kMaxParams + 8);
     if (!e) e = cudaMemcpy(dData.p, data.data(), sizeof(double) * n, cudaMemcpyHostToDevice);
@@ -681,6 +725,7 @@ struct imfit_model_s {
         y0 = params[x0Index[f] + 1];
       }
       comp_setup64(out[f], funcs[f].type, funcs[f].subsample, params + paramOffset[f], x0, y0);
+      comp_fast64(out[f], !refArith);
       if (funcs[f].type == F_EXPDISK3D || funcs[f].type == F_FERRERS3D) out[f].pad0 = k3++;
     }
   }
@@ -698,19 +743,28 @@ struct imfit_model_s {
   }
   cudaError_t evalGridN(const CompF64 *dC, int nC, const LosList64 &ll, double *model, long pitch,
                         const Grid64 &g0) {
-    // subsampled pixels: a table filled one warp per pixel (scratch reused by
-    // every grid; the launches are ordered on the one stream)
     Grid64 g = g0;
-    g.subHalf = g.isRegion ? (int)std::ceil(10.0 / g.frac) + 1 : 11;
-    cudaError_t e = dSub.reserve(std::max<size_t>(sub_table_size(g, nC), 1));
+    cudaError_t e = gridScratch(g, nC, 1);
     if (e) return e;
-    g.sub = dSub.p;
     if (ll.n == 0) return launch_eval64(dC, nC, model, pitch, g, nullptr, stream);
     const size_t need = (size_t)ll.n * g.nCols * g.nRows;
     e = dLos.reserve(need);
     if (!e) e = launch_los64(dC, ll, dLos.p, g, dLosFlag.p, stream);
     if (!e) e = launch_eval64(dC, nC, model, pitch, g, dLos.p, stream);
     return e;
+  }
+
+  // scratch of the subsampled pixels (reused by every grid; the launches are
+  // ordered on the one stream)
+  cudaError_t gridScratch(Grid64 &g, int nC, int nVec) {
+    g.subHalf = g.isRegion ? (int)std::ceil(10.0 / g.frac) + 1 : 11;
+    const size_t nLat = refArith ? 0 : lattice_size(g, nC);
+    cudaError_t e = dSub.reserve(std::max<size_t>(nVec * sub_table_size(g, nC), 1));
+    if (!e && nLat) e = dLattice.reserve(nVec * nLat);
+    if (e) return e;
+    g.sub = dSub.p;
+    g.lattice = nLat ? dLattice.p : nullptr;
+    return cudaSuccess;
   }
 
   // GetSingleFunctionImage (core/model_object.cpp:1241-1336): one function on
@@ -738,39 +792,24 @@ struct imfit_model_s {
     if (!e && ll.n) e = dLosFlag.reserve(1);
     if (!e && ll.n) e = cudaMemsetAsync(dLosFlag.p, 0, sizeof(int), stream);
     if (!e) e = cudaMemcpyAsync(dComps.p, &one, sizeof(CompF64), cudaMemcpyHostToDevice, stream);
-    Grid64 g{};
-    g.nCols = nModelCols;
-    g.nRows = nModelRows;
-    g.pc = doConv ? nPsfCols : 0;
-    g.pr = doConv ? nPsfRows : 0;
+    const Grid64 g = mainGrid();
     const bool ps = is_point_source(one.type);
     if (!e) e = evalGridN(dComps.p, 1, ll, dModel.p, nModelCols, g);
-    if (!e && doConv && !ps) e = conv64(dModel.p, nModelCols, nModelRows, Lx, Ly, dH.p, dSpec.p);
+    if (!e && doConv && !ps) e = conv64(dModel.p, nModelCols, nModelRows, Lx, Ly, dH.p, dSpec.p, 0, nModelRows);
     if (!e && ps) e = launch_point_sources64(dComps.p, 1, dModel.p, nModelCols, g, ps64, mainScales(&fi, 1), stream);
     for (Region *r : regions) {
       if (e) break;
-      Grid64 rg{};
-      rg.nCols = r->nModelCols;
-      rg.nRows = r->nModelRows;
-      rg.pc = r->nPsfCols;
-      rg.pr = r->nPsfRows;
-      rg.isRegion = 1;
-      rg.x1 = r->x1;
-      rg.y1 = r->y1;
-      rg.frac = 1.0 / r->scale;
-      rg.off = 0.5 * rg.frac - 0.5;
-      e = evalGridN(dComps.p, 1, ll, r->model.p, r->nModelCols, rg);
-      if (!e) e = conv64(r->model.p, r->nModelCols, r->nModelRows, r->Lx, r->Ly, r->H.p, r->spec.p);
+      RegionGrid &w = gridOf(*r);
+      const Grid64 rg = regionGrid(*r);
+      e = evalGridN(dComps.p, 1, ll, w.model.p, w.cols, rg);
+      if (!e) e = convRegion(*r, w.model.p, w.spec.p);
       if (!e && ps) {
         PsScales sc{};
         sc.s[0] = r->scale;
-        e = launch_point_sources64(dComps.p, 1, r->model.p, r->nModelCols, rg, r->ps64, sc, stream);
+        e = launch_point_sources64(dComps.p, 1, w.model.p, w.cols, rg, r->ps64, sc, stream);
         psScale[fi] = r->scale;
       }
-      if (!e)
-        e = launch_downsample64(r->model.p, r->nModelCols, r->nModelRows, r->nPsfCols, r->nPsfRows, dModel.p,
-                                nModelCols, nModelRows, doConv ? nPsfCols : 0, doConv ? nPsfRows : 0, r->x1, r->y1,
-                                r->scale, stream);
+      if (!e) e = downsample(*r, w.model.p, dModel.p);
     }
     DevBuf<double> tmp;
     if (!e) e = tmp.reserve(nDataVals);
@@ -859,13 +898,57 @@ struct imfit_model_s {
     return 0;
   }
 
+  // PSF convolution of nVec images (nCols x nRows each, in place); rows
+  // [row0, row1) of the result are formed.
   cudaError_t conv64(double *img, int nCols, int nRows, const FFTLen &fx, const FFTLen &fy, const double *H,
-                     double *spec) {
+                     double *spec, int row0, int row1, int nVec = 1) {
     const int nc = fx.L / 2 + 1;
-    cudaError_t e = launch_rows_r2c<double>(img, nCols, 0, nCols, nRows, spec, nc, 0, fx, 1, stream);
-    if (!e) e = launch_cols<double>(spec, nc, 0, nc, nRows, nRows, H, nc, fy, 1.0 / ((double)fx.L * fy.L), 1, 1, stream);
-    if (!e) e = launch_rows_c2r<double>(spec, nc, 0, nRows, img, nCols, 0, nCols, 1.0, fx, 1, stream);
+    const long is = (long)nCols * nRows, ss = (long)fy.L * nc;
+    cudaError_t e = launch_rows_r2c<double>(img, nCols, is, nCols, nRows, spec, nc, ss, fx, nVec, stream);
+    if (!e)
+      e = launch_cols<double>(spec, nc, ss, nc, nRows, row1, H, nc, fy, 1.0 / ((double)fx.L * fy.L), 1, nVec, stream);
+    if (!e)
+      e = launch_rows_c2r<double>(spec + 2 * (size_t)row0 * nc, nc, ss, row1 - row0, img + (size_t)row0 * nCols, nCols,
+                                  is, nCols, 1.0, fx, nVec, stream);
     return e;
+  }
+
+  // the region's convolution: the subpixel rows that are read back
+  cudaError_t convRegion(Region &r, double *model, double *spec, int nVec = 1) {
+    const RegionGrid &w = gridOf(r);
+    return conv64(model, w.cols, w.rows, w.Lx, w.Ly, w.H.p, spec, w.padR, w.padR + r.nRowsSub * r.scale, nVec);
+  }
+
+  cudaError_t downsample(Region &r, const double *model, double *mainModel, int nVec = 1) {
+    const RegionGrid &w = gridOf(r);
+    return launch_downsample64(model, w.cols, w.padC, w.padR, r.nColsSub, r.nRowsSub, mainModel, nModelCols,
+                               doConv ? nPsfCols : 0, doConv ? nPsfRows : 0, r.x1, r.y1, r.scale, stream, nVec,
+                               w.vals, nModelVals);
+  }
+
+  Grid64 mainGrid() const {
+    Grid64 g{};
+    g.nCols = nModelCols;
+    g.nRows = nModelRows;
+    g.pc = doConv ? nPsfCols : 0;
+    g.pr = doConv ? nPsfRows : 0;
+    return g;
+  }
+
+  Grid64 regionGrid(Region &r) const {
+    const RegionGrid &w = gridOf(r);
+    Grid64 g{};
+    g.nCols = w.cols;
+    g.nRows = w.rows;
+    g.pc = w.padC;
+    g.pr = w.padR;
+    g.isRegion = 1;
+    g.x1 = r.x1;
+    g.y1 = r.y1;
+    g.frac = 1.0 / r.scale;
+    g.off = 0.5 * g.frac - 0.5;
+    g.scale = r.scale;
+    return g;
   }
 
   // Interpolator tables for the point sources (built on first use, again
@@ -925,49 +1008,37 @@ struct imfit_model_s {
       if (e) return e;
       *hLosFlag = 0;
     }
-    Grid64 g{};
-    g.nCols = nModelCols;
-    g.nRows = nModelRows;
-    g.pc = doConv ? nPsfCols : 0;
-    g.pr = doConv ? nPsfRows : 0;
+    const Grid64 g = mainGrid();
     e = evalGrid(dC, dModel.p, nModelCols, g);
-    if (!e && doConv) e = conv64(dModel.p, nModelCols, nModelRows, Lx, Ly, dH.p, dSpec.p);
+    if (!e && doConv) e = conv64(dModel.p, nModelCols, nModelRows, Lx, Ly, dH.p, dSpec.p, 0, nModelRows);
     const int nC = (int)funcs.size();
     std::vector<int> all(nC);
     for (int c = 0; c < nC; c++) all[c] = c;
     if (!e && nPointSources) e = launch_point_sources64(dC, nC, dModel.p, nModelCols, g, ps64, mainScales(all.data(), nC), stream);
     for (Region *r : regions) {
       if (e) break;
-      Grid64 rg{};
-      rg.nCols = r->nModelCols;
-      rg.nRows = r->nModelRows;
-      rg.pc = r->nPsfCols;
-      rg.pr = r->nPsfRows;
-      rg.isRegion = 1;
-      rg.x1 = r->x1;
-      rg.y1 = r->y1;
-      rg.frac = 1.0 / r->scale;
-      rg.off = 0.5 * rg.frac - 0.5;
-      e = evalGrid(dC, r->model.p, r->nModelCols, rg);
-      if (!e) e = conv64(r->model.p, r->nModelCols, r->nModelRows, r->Lx, r->Ly, r->H.p, r->spec.p);
+      RegionGrid &w = gridOf(*r);
+      const Grid64 rg = regionGrid(*r);
+      e = evalGrid(dC, w.model.p, w.cols, rg);
+      if (!e) e = convRegion(*r, w.model.p, w.spec.p);
       if (!e && nPointSources) {
         PsScales sc{};
         for (int c = 0; c < nC; c++) sc.s[c] = r->scale;
-        e = launch_point_sources64(dC, nC, r->model.p, r->nModelCols, rg, r->ps64, sc, stream);
+        e = launch_point_sources64(dC, nC, w.model.p, w.cols, rg, r->ps64, sc, stream);
         for (int c = 0; c < nC; c++)
           if (is_point_source(funcs[c].type)) psScale[c] = r->scale;
       }
-      if (!e)
-        e = launch_downsample64(r->model.p, r->nModelCols, r->nModelRows, r->nPsfCols, r->nPsfRows, dModel.p,
-                                nModelCols, nModelRows, doConv ? nPsfCols : 0, doConv ? nPsfRows : 0, r->x1, r->y1,
-                                r->scale, stream);
+      if (!e) e = downsample(*r, w.model.p, dModel.p);
     }
     if (!e && losList.n) e = cudaMemcpyAsync(hLosFlag, dLosFlag.p, sizeof(int), cudaMemcpyDeviceToHost, stream);
-    if (!e && modelErrors && finalSetupDone)
-      e = launch_update_weights64(dModel.p, dMask.p, dWeight.p, nDataVals, nDataCols, nModelCols,
-                                  doConv ? nPsfRows : 0, doConv ? nPsfCols : 0, effGain, sky, nCombined * rnAduSq,
-                                  stream);
+    if (!e && modelErrors && finalSetupDone) e = updateWeights();
     return e;
+  }
+
+  cudaError_t updateWeights() {
+    return launch_update_weights64(dModel.p, dMask.p, dWeight.p, nDataVals, nDataCols, nModelCols,
+                                   doConv ? nPsfRows : 0, doConv ? nPsfCols : 0, effGain, sky, nCombined * rnAduSq,
+                                   stream);
   }
 
   // finish = false: only enqueued (the caller synchronises and then calls
@@ -1044,6 +1115,114 @@ struct imfit_model_s {
     return losCheck();
   }
 
+  // The 1 + nParams models of a finite-difference gradient as one batch: each
+  // stage one launch over all of them, and of a step's model only the
+  // components that the step changes evaluated (k_eval64, kDelta).  Their
+  // images and spectra are kept side by side, within kFdBytes.  One after
+  // another (fdSequential): beyond that, with line-of-sight components, and
+  // with point sources beside an oversampled region (whose pass changes the
+  // point sources' scale for the next model).
+  static constexpr size_t kFdBytes = 16ull << 30;
+  bool reserveFd(int nVec) {
+    const int nC = (int)funcs.size();
+    buildLosList();
+    if (losList.n || (nPointSources && !regions.empty())) return false;
+    size_t model = nModelVals, spec = doConv ? 2 * (size_t)Ly.L * (Lx.L / 2 + 1) : 0, rmodel = 0;
+    for (Region *r : regions) {
+      const RegionGrid &w = gridOf(*r);
+      rmodel = std::max(rmodel, (size_t)w.vals);
+      spec = std::max(spec, 2 * (size_t)w.Ly.L * (w.Lx.L / 2 + 1));
+    }
+    const size_t base = (size_t)nC * std::max(model, rmodel);
+    if (sizeof(double) * (nVec * (model + spec + rmodel) + base) > kFdBytes) return false;
+    cudaError_t e = dFdModel.reserve(nVec * model);
+    if (!e && spec) e = dFdSpec.reserve(nVec * spec);
+    if (!e && rmodel) e = dFdRegion.reserve(nVec * rmodel);
+    if (!e) e = dFdBase.reserve(base);
+    if (!e) e = dFdInvH.reserve(nVec);
+    if (!e) e = dFdChanged.reserve(nVec);
+    if (!e) e = dPart.reserve((size_t)nVec * kStatBlocks * 5);
+    if (e) cudaGetLastError();
+    return e == cudaSuccess;
+  }
+
+  // models of the vectors in dComps (all: their components, nVec x nC), then
+  // the statistic of vector 0 in dRes[0] and the gradient columns (chi^2) or
+  // the other vectors' statistics (Cash) after it.  dModel and the model-based
+  // weights are left as the last model's, as evaluating it last would.
+  cudaError_t fdBatch(const std::vector<CompF64> &all, const std::vector<double> &h, bool chi) {
+    const int nC = (int)funcs.size(), nP = (int)h.size(), nVec = nP + 1;
+    std::vector<unsigned> changed(nVec, 0u);
+    for (int v = 0; v < nVec; v++)
+      for (int c = 0; c < nC; c++)
+        if (memcmp(&all[(size_t)v * nC + c], &all[c], sizeof(CompF64)) != 0 || v == 0) changed[v] |= 1u << c;
+    std::vector<double> invh(nP);
+    for (int j = 0; j < nP; j++) invh[j] = 1.0 / h[j];
+    cudaError_t e = cudaMemcpyAsync(dFdChanged.p, changed.data(), sizeof(unsigned) * nVec, cudaMemcpyHostToDevice, stream);
+    if (!e && nP) e = cudaMemcpyAsync(dFdInvH.p, invh.data(), sizeof(double) * nP, cudaMemcpyHostToDevice, stream);
+    auto eval = [&](Grid64 g, double *model, long stride) {
+      cudaError_t er = gridScratch(g, nC, nVec);
+      if (!er)
+        er = launch_eval64(dComps.p, nC, model, g.nCols, g, nullptr, stream, nVec, stride, dFdBase.p, dFdChanged.p);
+      return er;
+    };
+    const Grid64 g = mainGrid();
+    if (!e) e = eval(g, dFdModel.p, nModelVals);
+    if (!e && doConv)
+      e = conv64(dFdModel.p, nModelCols, nModelRows, Lx, Ly, dH.p, dFdSpec.p, 0, nModelRows, nVec);
+    std::vector<int> ids(nC);
+    for (int c = 0; c < nC; c++) ids[c] = c;
+    for (int v = 0; v < nVec && nPointSources && !e; v++)
+      e = launch_point_sources64(dComps.p + (size_t)v * nC, nC, dFdModel.p + (size_t)v * nModelVals, nModelCols, g,
+                                 ps64, mainScales(ids.data(), nC), stream);
+    for (Region *r : regions) {
+      if (!e) e = eval(regionGrid(*r), dFdRegion.p, gridOf(*r).vals);
+      if (!e) e = convRegion(*r, dFdRegion.p, dFdSpec.p, nVec);
+      if (!e) e = downsample(*r, dFdRegion.p, dFdModel.p, nVec);
+    }
+    StatArgs64 a = statArgs(chi ? 0 : 1);
+    a.model = dFdModel.p;
+    a.modelErrors = modelErrors ? 1 : 0;  // each model's own weights, formed as they are read
+    if (!e) e = launch_statistic64(a, dPart.p, dRes.p, stream, chi ? 1 : nVec, nModelVals);
+    if (!e && chi) e = launch_fd_dot64(a, nModelVals, nP, dFdInvH.p, dPart.p, dRes.p + 1, stream);
+    if (!e)
+      e = cudaMemcpyAsync(dModel.p, dFdModel.p + (size_t)nP * nModelVals, sizeof(double) * nModelVals,
+                          cudaMemcpyDeviceToDevice, stream);
+    if (!e && modelErrors) e = updateWeights();
+    return e;
+  }
+
+  cudaError_t fdSequential(const std::vector<double> &h, bool chi) {
+    const int nC = (int)funcs.size(), nP = (int)h.size();
+    StatArgs64 a = statArgs(chi ? 0 : 1);
+    cudaError_t e = dFdModel.reserve(chi ? 2 * nModelVals : 1);
+    if (!e) e = dFdInvH.reserve(nP + 1);
+    std::vector<double> invh(nP);
+    for (int j = 0; j < nP; j++) invh[j] = 1.0 / h[j];
+    if (!e && nP) e = cudaMemcpyAsync(dFdInvH.p, invh.data(), sizeof(double) * nP, cudaMemcpyHostToDevice, stream);
+    if (!e) e = enqueueModel(dComps.p);
+    if (!e) e = launch_statistic64(a, dPart.p, dRes.p, stream);
+    StatArgs64 two = a;  // models 0 and 1 + j side by side, each with its own model-based weights
+    two.model = dFdModel.p;
+    two.modelErrors = modelErrors ? 1 : 0;
+    auto keep = [&](int slot) {
+      return cudaMemcpyAsync(dFdModel.p + (size_t)slot * nModelVals, dModel.p, sizeof(double) * nModelVals,
+                             cudaMemcpyDeviceToDevice, stream);
+    };
+    if (!e && chi) e = keep(0);
+    for (int j = 0; j < nP && !e; j++) {
+      e = enqueueModel(dComps.p + (size_t)(j + 1) * nC);
+      if (e) break;
+      if (chi) {
+        e = keep(1);
+        if (!e) e = launch_fd_dot64(two, nModelVals, 1, dFdInvH.p + j, dPart.p, dRes.p + 1 + j, stream);
+      } else {
+        e = launch_statistic64(a, dPart.p, dRes.p + 1 + j, stream);
+      }
+    }
+    return e;
+  }
+
   // statistic + FD gradient (1 + nParams plain evaluations)
   int fdGradient(const double *params, double *stat, double *grad) {
     if (!finalSetupDone) return fail(IMFIT_E_STATE, "FinalSetupForFitting not called");
@@ -1051,6 +1230,19 @@ struct imfit_model_s {
     if (st) return st;
     const int nP = nParamsTot, nC = (int)funcs.size();
     const double eps = sqrt(2.2204460e-16);  // MP_MACHEP0 (solvers/mpfit.h)
+    // A step is 1.5e-8 of the parameter, so the gradient holds every model's
+    // rounding errors times 7e7: evaluated another way, or convolved with
+    // another FFT length, it moves by 1e-8 to 1e-6 of itself.  The entry point
+    // that stands for the reference's differences therefore keeps the
+    // reference's expressions and padding, bit for bit, and gains from
+    // batching and from skipping what a step does not change.
+    struct Ref {
+      bool &f;
+      explicit Ref(bool &x) : f(x) { f = true; }
+      ~Ref() { f = false; }
+    } ref(refArith);
+    for (Region *r : regions)
+      if ((st = makeRegionGrid(*r, r->full, false))) return st;
     std::vector<CompF64> all((size_t)(nP + 1) * nC);
     std::vector<double> x(params, params + nP), h(nP);
     setupComps(x.data(), all.data());
@@ -1065,21 +1257,13 @@ struct imfit_model_s {
     }
     cudaError_t e = dComps.reserve(all.size());
     if (!e) e = cudaMemcpyAsync(dComps.p, all.data(), sizeof(CompF64) * all.size(), cudaMemcpyHostToDevice, stream);
+    if (e) return cuda_fail(e, "FD gradient");
     const bool chi = !useCash;
-    StatArgs64 a = statArgs(chi ? 0 : 1);
-    if (!e) e = enqueueModel(dComps.p);
-    if (!e) e = launch_statistic64(a, dPart.p, dRes.p, stream);
-    if (chi && !e) e = launch_deviates64(statArgs(0), dDev.p, nullptr, stream);
-    for (int j = 0; j < nP && !e; j++) {
-      e = enqueueModel(dComps.p + (size_t)(j + 1) * nC);
-      if (e) break;
-      if (chi) {
-        e = launch_deviates64(statArgs(0), dDev2.p, nullptr, stream);
-        if (!e) e = launch_fd_dot64(dDev.p, dDev2.p, a.nz, 1.0 / h[j], dPart.p, dRes.p + 1 + j, stream);
-      } else {
-        e = launch_statistic64(a, dPart.p, dRes.p + 1 + j, stream);
-      }
-    }
+    const bool batch = reserveFd(nP + 1);
+    if (batch)
+      e = fdBatch(all, h, chi);
+    else
+      e = fdSequential(h, chi);
     double *hb = pinned(nP + 1);
     if (!e) e = cudaMemcpyAsync(hb, dRes.p, sizeof(double) * (nP + 1), cudaMemcpyDeviceToHost, stream);
     if (!e) e = cudaStreamSynchronize(stream);
