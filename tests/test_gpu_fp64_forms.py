@@ -140,3 +140,22 @@ def test_batched_finite_differences(gpu, oracle_mod, stat, region):
     left = g.get_model_image()
     g.create_model_image(last)
     assert normwise(left, g.get_model_image()) < 1e-10
+
+
+@pytest.mark.parametrize("n", [1.0, 2.0, 3.0, 2.5, 0.4])
+def test_ferrers_indices(gpu, oracle_mod, n):
+    p = [25.3, 22.8, 35.0, 70.0, 40.0, 2.0, 14.0, 0.5, 0.3, n]
+    g, o = _images(gpu, oracle_mod, ["FerrersBar3D"], p, 50, 45)
+    # the integrals are adaptive to 1e-6; below n = 1 the density's edge is steep
+    assert np.max(np.abs(g - o)) <= 1e-12 * np.max(o)
+
+
+# (0.5, 0.02, 90) holds pixels whose whole integrand is denormal, which no
+# form integrates within the device's list of subintervals (refused)
+@pytest.mark.parametrize("n,z0,inc", [(1.0, 2.0, 85.0), (0.5, 0.02, 89.0), (100.0, 3.0, 0.0), (3.0, 0.7, 40.0)])
+def test_disk_vertical_profiles(gpu, oracle_mod, n, z0, inc):
+    """Thin disks reach z / (alpha z_0) > 100, where the reference switches to
+    the asymptote, and values at the bottom of the FP64 range."""
+    p = [25.3, 22.8, 35.0, inc, 4.0, 6.0, n, z0]
+    g, o = _images(gpu, oracle_mod, ["ExponentialDisk3D"], p, 50, 45)
+    assert np.max(np.abs(g - o)) <= 1e-12 * np.max(o)
