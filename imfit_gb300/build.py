@@ -23,6 +23,7 @@ UNITS = [
     ("k_fft.cu", []),
     ("k_fast.cu", []),
     ("k_cols32.cu", []),
+    ("k_cols2.cu", []),
     ("model_object.cpp", ["-x", "cu"]),
     ("k_noalloc.cu", ["--fmad=false"]),
     ("lm.cpp", []),

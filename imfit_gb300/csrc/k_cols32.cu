@@ -18,8 +18,7 @@
 //     and written back with 16-byte vector stores;
 //   * the FFT passes read their twiddles from the shared-memory copy.
 // Rows at or beyond nRowsIn are the implicit zero padding and are never read.
-#include "kernels.h"
-#include "fft.cuh"
+#include "cols2.cuh"
 
 namespace imfit {
 
@@ -27,10 +26,6 @@ namespace {
 
 __device__ __forceinline__ unsigned smem_addr(const void *p) {
   return (unsigned)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr(dst)), "l"(src) : "memory");
 }
 
 __device__ __forceinline__ void cp_async8(void *dst, const void *src) {
@@ -427,30 +422,43 @@ cudaError_t launch_mode(int cpb, cplx<float> *s, long pitch, long batch, int nCo
 
 // Column pass of a ragged cutout set: CTA t serves column group g of spectrum
 // `line` of the slot that owns t (each cutout its own lengths and pitch).
-constexpr int kRagCpb = kRagColsPerCta;
-__global__ void __launch_bounds__(256) k_rag_cols(RagArgs r) {
+// Cutout lengths nearly all have the two-pass form (cols2.cuh); entries without
+// one take the fused multi-pass group.
+__global__ void __launch_bounds__(kTwoPassThreads, 4) k_rag_cols(RagArgs r) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_wait();
   const int t = blockIdx.x;
   const int k = rag_slot(r.start, r.K, t);
   const RagEntry &E = r.ent[r.act[k]];
   const int local = t - r.start[k];
-  const int line = local / E.colGroups, g = local - line * E.colGroups;
-  cplx<float> *spec = r.spec + (r.lines == 1 ? E.specOff : (long)r.lines * E.specOff + (long)line * E.specSize);
+  const int line = local / E.colGroups, c0 = (local - line * E.colGroups) * E.cpb, nCols = E.Lx / 2 + 1;
+  cplx<float> *spec = r.spec + (long)r.lines * E.specOff + (long)line * E.specSize;
   const float scale = 1.f / ((float)E.Lx * (float)E.Ly);
-  if (E.colPlanI.tw)
-    cols_group_fused<1, kRagCpb>(smem_raw, spec, E.pitch, E.Lx / 2 + 1, E.winRows, E.nDataRows, r.H + E.hOff,
-                                 E.pitch, E.colPlan, E.colPlanI, scale, g * kRagCpb);
+  if (E.colTwo.R1)
+    cols_two_pass(smem_raw, spec + c0, E.pitch, min(E.cpb, nCols - c0), E.winRows, E.nDataRows, r.H + E.hOff + c0,
+                  E.pitch, E.colTwo, scale, scale, E.cpb);
+  else if (E.colPlanI.tw)
+    cols_group_fused<1, kRagColsPerCta>(smem_raw, spec, E.pitch, nCols, E.winRows, E.nDataRows, r.H + E.hOff, E.pitch,
+                                        E.colPlan, E.colPlanI, scale, c0);
   else
-    cols_group<1, kRagCpb>(smem_raw, spec, E.pitch, E.Lx / 2 + 1, E.winRows, E.nDataRows, r.H + E.hOff, E.pitch,
-                           E.colPlan, scale, g * kRagCpb);
+    cols_group<1, kRagColsPerCta>(smem_raw, spec, E.pitch, nCols, E.winRows, E.nDataRows, r.H + E.hOff, E.pitch,
+                                  E.colPlan, scale, c0);
 }
 
-cudaError_t launch_rag_cols(const RagArgs &r, int total, int maxLy, cudaStream_t st) {
+void rag_cols_shape(const RagEntry &E, size_t &smem, int &threads) {
+  if (E.colTwo.R1) {
+    smem = std::max(smem, cols2_smem(E.colTwo, E.cpb));
+    threads = std::max(threads, (E.cpb * E.colTwo.R1 + 31) / 32 * 32);
+  } else {
+    smem = std::max(smem, std::max(cols32_smem(E.Ly, kRagColsPerCta), cols32_fused_smem(E.Ly, kRagColsPerCta)));
+    threads = std::max(threads, 128);
+  }
+}
+
+cudaError_t launch_rag_cols(const RagArgs &r, int total, size_t smem, int threads, cudaStream_t st) {
   if (total <= 0) return cudaSuccess;
   allow_max_smem((const void *)k_rag_cols);
-  const size_t sm = std::max(cols32_smem(maxLy, kRagCpb), cols32_fused_smem(maxLy, kRagCpb));
-  return launch_pdl(k_rag_cols, dim3(total), dim3(128), sm, st, r);
+  return launch_pdl(k_rag_cols, dim3(total), dim3(threads), smem, st, r);
 }
 
 // the fused form: both plans' twiddles and the two FFT buffers
@@ -466,6 +474,9 @@ cudaError_t launch_cols32(void *spec, long pitch, long batch, int nColsC, int nR
                           long hPitch, const FFTLen &Ly, float scale, int mode, int nBatch, cudaStream_t st, int cpb,
                           long hBatch, int hDiv, const int *hMap, int threads) {
   if ((pitch & 1) || (hPitch & 1) || (Ly.full.n & 1) || mode < 1 || mode > 2) return cudaErrorInvalidValue;
+  if (Ly.full.two.R1 && (long)nColsC * nBatch >= kTwoPassColumns)
+    return launch_cols2(spec, pitch, batch, nColsC, nRowsIn, nRowsOut, H, hPitch, Ly.full.two, scale, mode, nBatch, st,
+                        cpb, hBatch, hDiv, hMap);
   int optin = 0, dev = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -501,6 +512,7 @@ cudaError_t launch_cols32(void *spec, long pitch, long batch, int nColsC, int nR
 }
 
 void cols32_prepare_kernels() {
+  cols2_prepare_kernels();
   allow_max_smem((const void *)k_cols32<1, 1>);
   allow_max_smem((const void *)k_cols32<1, 2>);
   allow_max_smem((const void *)k_cols32<1, 4>);

@@ -2466,8 +2466,8 @@ size_t rag_jtwj_smem(int maxM, int nD, int nP, int maxCols) {
 // derivative spectra; starts/totals are the slots' prefix sums and totals per
 // kind of work.
 cudaError_t rag_jtwj(const FastArgs &a, RagArgs r, cplx<float> *dspec, const int *const starts[kRagWorkKinds],
-                     const int totals[kRagWorkKinds], const int *slot, int nD, int maxM, int maxLy, int maxCols,
-                     double *alpha, double *beta, double *stat, cudaStream_t st) {
+                     const int totals[kRagWorkKinds], const int *slot, int nD, int maxM, size_t colSmem, int colThreads,
+                     int maxCols, double *alpha, double *beta, double *stat, cudaStream_t st) {
   const int K = r.K;
   if (K <= 0) return cudaSuccess;
   cudaError_t e;
@@ -2482,7 +2482,7 @@ cudaError_t rag_jtwj(const FastArgs &a, RagArgs r, cplx<float> *dspec, const int
     return e;
   r.start = starts[kRagCols];
   r.lines = 1;
-  if ((e = launch_rag_cols(r, totals[kRagCols], maxLy, st))) return e;
+  if ((e = launch_rag_cols(r, totals[kRagCols], colSmem, colThreads, st))) return e;
   r.start = starts[kRagDataRows];
   allow_max_smem((const void *)k_rag_model_rows);
   if ((e = launch_pdl(k_rag_model_rows, dim3(totals[kRagDataRows]), dim3(kRagRowThreads),
@@ -2499,7 +2499,7 @@ cudaError_t rag_jtwj(const FastArgs &a, RagArgs r, cplx<float> *dspec, const int
       return e;
     rd.start = starts[kRagDerivCols];
     rd.lines = nD;
-    if ((e = launch_rag_cols(rd, totals[kRagDerivCols], maxLy, st))) return e;
+    if ((e = launch_rag_cols(rd, totals[kRagDerivCols], colSmem, colThreads, st))) return e;
   }
   rd.start = starts[kRagDataRows];
   allow_max_smem((const void *)k_rag_jtwj_rows);

@@ -389,7 +389,7 @@ int smooth_candidates(int n, bool even, int count, double maxRatio, int *out) {
 // read consecutive entries (no shared-memory bank conflicts once staged);
 // each value is the one a single table exp(-2 pi i m / n) holds at
 // m = r k n / (Ns R).
-static cudaError_t table_create(FFTTable &t, int n, int variant, bool reversed = false) {
+static cudaError_t table_create(FFTTable &t, int n, int variant, bool reversed, bool twoPass) {
   t.n = n;
   t.npass = radix_schedule(n, t.radix, variant);
   if (t.npass < 0) return cudaErrorInvalidValue;
@@ -421,18 +421,36 @@ static cudaError_t table_create(FFTTable &t, int n, int variant, bool reversed =
   if (e) return e;
   e = cudaMemcpy(t.tw64, w64.data(), sizeof(double) * 2 * (size_t)n, cudaMemcpyHostToDevice);
   if (e) return e;
-  return cudaMemcpy(t.tw32, w32.data(), sizeof(float) * 2 * (size_t)n, cudaMemcpyHostToDevice);
+  e = cudaMemcpy(t.tw32, w32.data(), sizeof(float) * 2 * (size_t)n, cudaMemcpyHostToDevice);
+  if (e || !twoPass) return e;
+  TwoPass &f = t.two;
+  if (!two_pass_factors(n, f.R1, f.R2)) return cudaSuccess;
+  const int P = two_pass_pitch(f.R2);
+  std::vector<float> w2(2 * (size_t)two_pass_table(f.R1, f.R2), 0.f);
+  for (int k1 = 0; k1 < f.R1; k1++)
+    for (int n2 = 0; n2 < f.R2; n2++) {
+      const size_t m = (size_t)k1 * n2, a = (size_t)k1 * P + n2;
+      w2[2 * a] = (float)full[2 * m];
+      w2[2 * a + 1] = (float)full[2 * m + 1];
+    }
+  cplx<float> *d = nullptr;
+  e = cudaMalloc(&d, sizeof(float) * w2.size());
+  if (!e) e = cudaMemcpy(d, w2.data(), sizeof(float) * w2.size(), cudaMemcpyHostToDevice);
+  f.t = d;
+  if (e) f.R1 = f.R2 = 0;
+  return e;
 }
 
 cudaError_t fftlen_create(FFTLen &L, int len, int variant) {
   L.L = len;
   L.variant = variant;
-  cudaError_t e = table_create(L.full, len, variant);
+  // the two-pass form for the fast path's columns, whatever their radix order
+  cudaError_t e = table_create(L.full, len, variant, false, variant != kRadixPlain);
   if (e) return e;
-  e = table_create(L.fullRev, len, variant, true);
+  e = table_create(L.fullRev, len, variant, true, false);
   if (e) return e;
   if (len % 2 == 0) {
-    e = table_create(L.half, len / 2, variant);
+    e = table_create(L.half, len / 2, variant, false, false);
     if (e) return e;
     const int M = len / 2;
     std::vector<double> w64(2 * (size_t)(M + 1));
@@ -459,6 +477,8 @@ static void table_destroy(FFTTable &t) {
   if (t.tw64) cudaFree(t.tw64);
   if (t.tw32) cudaFree(t.tw32);
   t.tw64 = t.tw32 = nullptr;
+  if (t.two.t) cudaFree(const_cast<cplx<float> *>(t.two.t));
+  t.two = TwoPass{};
 }
 
 void fftlen_destroy(FFTLen &L) {

@@ -5,7 +5,7 @@
 #include <cstdint>
 #include <utility>
 #include "common.cuh"
-#include "fft.cuh"
+#include "fft2.cuh"
 #include "psf_interp.cuh"
 
 namespace imfit {
@@ -65,6 +65,8 @@ struct FFTTable {
   int radix[16] = {0};
   void *tw64 = nullptr;  // n complex doubles: exp(-2 pi i k / n)
   void *tw32 = nullptr;  // n complex floats
+  // two-pass form (fft2.cuh) where n has one
+  TwoPass two;
 };
 
 // A padded real line length L (even): the half-length complex transform used
@@ -113,6 +115,17 @@ cudaError_t launch_cols(void *spec, long pitch, long batch, int nColsC, int nRow
 cudaError_t launch_cols32(void *spec, long pitch, long batch, int nColsC, int nRowsIn, int nRowsOut, const void *H,
                           long hPitch, const FFTLen &Ly, float scale, int mode, int nBatch, cudaStream_t st,
                           int cpb = 0, long hBatch = 0, int hDiv = 1, const int *hMap = nullptr, int threads = 0);
+// The same in two register passes for lengths that have the form (k_cols2.cu;
+// launch_cols32 chooses); kTwoPassThreads: most threads of a CTA.
+constexpr int kTwoPassThreads = 160;
+// fewest columns of a launch that takes it: about two CTAs of four columns per SM
+constexpr long kTwoPassColumns = 1200;
+cudaError_t launch_cols2(void *spec, long pitch, long batch, int nColsC, int nRowsIn, int nRowsOut, const void *H,
+                         long hPitch, const TwoPass &f, float scale, int mode, int nBatch, cudaStream_t st, int cpb,
+                         long hBatch, int hDiv, const int *hMap);
+int cols2_cpb(const TwoPass &f, int most);
+size_t cols2_smem(const TwoPass &f, int cpb);
+void cols2_prepare_kernels();
 size_t cols32_smem(int Ly, int cpb);
 size_t cols32_fused_smem(int Ly, int cpb);
 void cols32_prepare_kernels();
@@ -364,7 +377,8 @@ cudaError_t fast_jtwj(const FastPlan &p, const FastArgs &a, const JtwjArgs &J, i
 // and every stage of an evaluation is ONE launch over all active cutouts --
 // a flat grid whose CTA t serves the slot k with start[k] <= t < start[k+1]
 // (binary search over the prefix sums of the slots' work counts).
-// spectrum columns per CTA of a cutout set's column pass
+// spectrum columns per CTA of a cutout set's column pass where the length has
+// no two-pass form
 constexpr int kRagColsPerCta = 4;
 
 struct RagEntry {
@@ -382,6 +396,8 @@ struct RagEntry {
   FFTPlan<float> rowPlan;    // Lx/2-point complex transform (rows)
   FFTPlan<float> colPlan;    // Ly-point transform (columns)
   FFTPlan<float> colPlanI;   // the same radices reversed (the column pass's inverse half; tw null: unfused)
+  TwoPass colTwo;            // the two-pass form (R1 0: none)
+  int cpb;                   // columns of one column group
   const cplx<float> *twL;    // Lx split twiddles
 };
 
@@ -415,11 +431,13 @@ __device__ __forceinline__ int rag_slot(const int *start, int K, int t) {
 enum RagWork { kRagWinRows = 0, kRagDataRows = 1, kRagCols = 2, kRagDerivCols = 3, kRagWorkKinds = 4 };
 
 cudaError_t rag_jtwj(const FastArgs &a, RagArgs r, cplx<float> *dspec, const int *const starts[kRagWorkKinds],
-                     const int totals[kRagWorkKinds], const int *slot, int nD, int maxM, int maxLy, int maxCols,
-                     double *alpha, double *beta, double *stat, cudaStream_t st);
+                     const int totals[kRagWorkKinds], const int *slot, int nD, int maxM, size_t colSmem, int colThreads,
+                     int maxCols, double *alpha, double *beta, double *stat, cudaStream_t st);
 // shared memory of the ragged derivative and row-product kernels
 size_t rag_jtwj_smem(int maxM, int nD, int nP, int maxCols);
-cudaError_t launch_rag_cols(const RagArgs &r, int total, int maxLy, cudaStream_t st);
+// smem, threads: the largest any entry needs (rag_cols_shape)
+cudaError_t launch_rag_cols(const RagArgs &r, int total, size_t smem, int threads, cudaStream_t st);
+void rag_cols_shape(const RagEntry &E, size_t &smem, int &threads);
 size_t fast_jtwj_smem(const FastPlan &p, int nD, int nP);
 cudaError_t fast_forward(const FastPlan &p, const FastArgs &a, int nBatch, bool wantGrad, cudaStream_t st);
 // one-time kernel attribute set-up (call before any stream capture)

@@ -343,7 +343,9 @@ struct imfit_model_s {
     std::vector<RagEntry> ent;
     std::map<int, std::unique_ptr<FFTLen>> lens;
     long totalPix = 0, totalSpec = 0, totalRows = 0, totalH = 0;
-    int maxM = 0, maxLy = 0, maxCols = 0;
+    int maxM = 0, maxCols = 0;
+    size_t colSmem = 0;  // launch shape of the column pass
+    int colThreads = 0;
     std::vector<int> work;  // act, then the prefix arrays, uploaded per evaluation
     ~RagSet() {
       for (auto &kv : lens) fftlen_destroy(*kv.second);
@@ -1773,6 +1775,7 @@ struct imfit_model_s {
       }
       for (int cpb : {1, 2, 4, 8}) {
         for (int nt : {0, 128, 256, 512}) {
+          if (nt && Fy.full.two.R1 && (long)(Fx.L / 2 + 1) * B >= kTwoPassColumns) continue;  // it sets its own
           FastTune t = bestT;
           t.colCpb = cpb;
           t.colThreads = nt;
@@ -2107,7 +2110,8 @@ struct imfit_model_s {
     RagSet &R = rag;
     R.ent.assign(nImg, RagEntry{});
     R.totalPix = R.totalSpec = R.totalRows = 0;
-    R.maxM = R.maxLy = R.maxCols = 0;
+    R.maxM = R.maxCols = R.colThreads = 0;
+    R.colSmem = 0;
     std::vector<long> psfOff(nImg);
     long np = 0;
     for (int i = 0; i < nImg; i++) {
@@ -2127,7 +2131,6 @@ struct imfit_model_s {
       E.Ly = smooth_size(E.winRows, true);
       if (E.Lx / 2 > 4096 || E.Ly > 4096) return fail(IMFIT_E_UNSUPPORTED, "cutout too large for the fast path");
       E.pitch = even_pitch(E.Lx);
-      E.colGroups = (E.Lx / 2 + 1 + kRagColsPerCta - 1) / kRagColsPerCta;
       E.specSize = (long)E.Ly * E.pitch;
       E.specOff = R.totalSpec;
       E.hOff = R.totalSpec;  // one PSF spectrum per cutout, same geometry
@@ -2137,7 +2140,6 @@ struct imfit_model_s {
       R.totalSpec += E.specSize;
       R.totalRows += nr;
       R.maxM = std::max(R.maxM, E.Lx / 2);
-      R.maxLy = std::max(R.maxLy, E.Ly);
       R.maxCols = std::max(R.maxCols, nc);
     }
     R.totalH = R.totalSpec;
@@ -2191,6 +2193,10 @@ struct imfit_model_s {
       E.colPlan = plan(fy->full);
       E.colPlanI = plan(fy->fullRev);
       if (E.colPlan.npass < 2) E.colPlanI.tw = nullptr;  // a single pass: the unfused column group
+      E.colTwo = fy->full.two;
+      E.cpb = E.colTwo.R1 ? cols2_cpb(E.colTwo, 8) : kRagColsPerCta;
+      E.colGroups = (E.Lx / 2 + 1 + E.cpb - 1) / E.cpb;
+      rag_cols_shape(E, R.colSmem, R.colThreads);
       E.twL = reinterpret_cast<const cplx<float> *>(fx->twL32);
     }
     e = dRagEnt.reserve(nImg);
@@ -2305,7 +2311,7 @@ struct imfit_model_s {
     }
     r.start = starts[kRagWinRows];
     e = rag_jtwj(a, r, reinterpret_cast<cplx<float> *>(dRagDSpec.p), starts, totals, dRagSlot.p, ragNDeriv, R.maxM,
-                 R.maxLy, R.maxCols, dRagA.p, dRagB.p, dRagS.p, stream);
+                 R.colSmem, R.colThreads, R.maxCols, dRagA.p, dRagB.p, dRagS.p, stream);
     if (e) return cuda_fail(e, "cutout-set J^T J launch");
     e = cudaMemcpyAsync(stats, dRagS.p, sizeof(double) * K, cudaMemcpyDeviceToHost, stream);
     if (!e) e = cudaMemcpyAsync(alpha, dRagA.p, sizeof(double) * (size_t)K * nP * nP, cudaMemcpyDeviceToHost, stream);
