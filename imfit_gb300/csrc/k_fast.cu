@@ -1454,6 +1454,7 @@ __global__ void __launch_bounds__(512) k_fast_deriv_r2c(FastArgs a, WinDesc w, F
                                                         const cplx<float> *__restrict__ twL,
                                                         const int *__restrict__ slot, int nD, int win) {
   extern __shared__ __align__(16) unsigned char smem[];
+  pdl_wait();
   const int b = blockIdx.y, row = blockIdx.x;
   const int M = plan.n, ls = M + 1;
   CompF32 *sc = reinterpret_cast<CompF32 *>(smem);
@@ -1499,6 +1500,7 @@ __global__ void __launch_bounds__(512) k_fast_deriv_r2c(FastArgs a, WinDesc w, F
   }
   __syncthreads();
   cplx<float> *Z = block_fft(bufA, bufB, plan, nD, ls, 1, -1, false);
+  pdl_trigger();
   cplx<float> *out = w.spec + (long)b * nD * w.specBatch + (long)row * w.specPitch;
   const FastDiv byM1(M + 1);
   for (int idx = threadIdx.x; idx < nD * (M + 1); idx += blockDim.x) {
@@ -1635,6 +1637,73 @@ __device__ __forceinline__ void jtwj_gram(const float *U, long uStride, const in
   }
 }
 
+// The model image from the derivative images: every pixel function is linear
+// in its amplitude (TiltedSkyPlane in all three parameters) and so is the
+// convolution, so the convolved model is sum over (line, value) of value times
+// line, plus the constant backgrounds (and the point sources).  No forward
+// pass is needed beside the derivative images: of the 1024 x 1024 benchmark
+// model's evaluation it took 95 of 500 us (model rows, columns, inverse rows,
+// the region's three stages), of a 256-cutout round 445 of 3490.
+//
+// The list sits in the space that the parameters leave of ss (kMaxParams
+// integers): count, then (line, value) pairs; count -1 where they do not fit
+// (then every pixel walks the components).
+//
+// Number of linear parameters of a type, the first one's offset; their
+// values are CompF32::s0 (TiltedSkyPlane: s0, s1, s2).
+__device__ __forceinline__ int n_linear(int t, int &first) {
+  first = t == F_SERSIC ? 3 : (t == F_TILTEDSKY ? 0 : 2);
+  return t == F_TILTEDSKY ? 3 : (t == F_SERSIC || t == F_EXP || t == F_GRING || t == F_MOFFAT || t == F_GAUSS);
+}
+// by the first warp, one lane per component (at most 32)
+__device__ __forceinline__ void find_amplitudes(const FastArgs &a, int b, const int *__restrict__ slot, int *ss) {
+  static_assert(kMaxComponents <= 32, "one lane per component");
+  if (threadIdx.x >= 32) return;
+  const int lane = threadIdx.x;
+  int n = 0, first = 0, off = 0;
+  float v[3] = {0.f, 0.f, 0.f};
+  if (lane < a.nComp) {
+    const CompF32 &cc = a.comps[b * a.nComp + lane];
+    n = n_linear(cc.type, first);
+    off = cc.paramOffset + first;
+    v[0] = cc.s0;
+    v[1] = cc.s1;
+    v[2] = cc.s2;
+  }
+  int at = n;  // inclusive scan
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, at, o);
+    if (lane >= o) at += t;
+  }
+  const int total = __shfl_sync(0xffffffffu, at, 31);
+  const bool fits = a.nParams + 1 + 2 * total <= kMaxParams;
+  int *list = ss + a.nParams;
+  if (lane == 0 && a.nParams < kMaxParams) list[0] = fits ? total : -1;
+  if (fits)
+    for (int q = 0; q < n; q++) {
+      list[1 + 2 * (at - n + q)] = slot[off + q];
+      list[2 + 2 * (at - n + q)] = __float_as_int(v[q]);
+    }
+}
+// model value of a column: bg plus the lines at u (line j at u[j * uStride])
+__device__ __forceinline__ float model_from_lines(const FastArgs &a, int b, const int *ss, const float *u, long uStride,
+                                                  float m) {
+  const int *list = ss + a.nParams;
+  const int n = a.nParams < kMaxParams ? list[0] : -1;
+  if (n >= 0) {
+    for (int i = 0; i < n; i++) m = fmaf(__int_as_float(list[2 + 2 * i]), u[list[1 + 2 * i] * uStride], m);
+    return m;
+  }
+  for (int c = 0; c < a.nComp; c++) {
+    const CompF32 &cc = a.comps[b * a.nComp + c];
+    int first;
+    const int k = n_linear(cc.type, first);
+    for (int q = 0; q < k; q++)
+      m = fmaf(q == 0 ? cc.s0 : (q == 1 ? cc.s1 : cc.s2), u[ss[cc.paramOffset + first + q] * uStride], m);
+  }
+  return m;
+}
+
 // One CTA per (data row, parameter vector): inverse row FFT of the nD
 // convolved derivative rows, the per-pixel Jacobian rows u_j = q dM/dtheta_j
 // (region pixels from the downsampled region derivatives, background
@@ -1649,12 +1718,14 @@ __global__ void __launch_bounds__(1024) k_fast_jtwj_rows(FastArgs a, FastGeom g,
                                                         const int *__restrict__ slot, int nD,
                                                         float2 *__restrict__ part, float *__restrict__ jac) {
   extern __shared__ __align__(16) unsigned char smem[];
+  pdl_wait();
   const int b = blockIdx.y, row = blockIdx.x;
   const int M = plan.n, ls = M + 1, nP = a.nParams, nc = g.nDataCols;
   int *ss = reinterpret_cast<int *>(smem);
   cplx<float> *bufA = reinterpret_cast<cplx<float> *>(ss + kMaxParams);
   cplx<float> *bufB = bufA + nD * ls;
   for (int i = threadIdx.x; i < nP; i += blockDim.x) ss[i] = slot[i];
+  find_amplitudes(a, b, slot, ss);
   if (a.dataStride) {  // image stack: this entry's data and weights
     const long img = a.entry ? a.entry[b] : b;
     a.data += img * a.dataStride;
@@ -1681,10 +1752,6 @@ __global__ void __launch_bounds__(1024) k_fast_jtwj_rows(FastArgs a, FastGeom g,
   const long nPix = (long)g.nDataRows * nc;
   for (int col = threadIdx.x; col < nc; col += blockDim.x) {
     const long zi = (long)row * nc + col;
-    const float m = a.modelOut[(long)b * nPix + zi];
-    float dev, q;
-    deviate_slope(a, zi, m, dev, q);
-    const float cnt = a.count ? a.count[zi] : 1.f;
     bool inReg = false;
     long ri = 0;
     if (g.hasRegion) {
@@ -1695,10 +1762,16 @@ __global__ void __launch_bounds__(1024) k_fast_jtwj_rows(FastArgs a, FastGeom g,
       }
     }
     const long rStride = (long)g.rRows * g.rCols;
-    for (int j = 0; j < nD; j++) {
-      float *u = Zr + j * uStride + col;
-      *u = q * (inReg ? regDeriv[((long)b * nD + j) * rStride + ri] : *u);
-    }
+    if (inReg)
+      for (int j = 0; j < nD; j++) Zr[j * uStride + col] = regDeriv[((long)b * nD + j) * rStride + ri];
+    float m = model_from_lines(a, b, ss, Zr + col, uStride, a.bgLevel[2 * b + (inReg ? 1 : 0)]);
+    if constexpr (PS)
+      m += inReg ? ps_region(a, g.rScale, b, row, col, 0.f, nullptr) / (float)(g.rScale * g.rScale)
+                 : ps_main(a, b, row, col, 0.f, nullptr);
+    float dev, q;
+    deviate_slope(a, zi, m, dev, q);
+    const float cnt = a.count ? a.count[zi] : 1.f;
+    for (int j = 0; j < nD; j++) Zr[j * uStride + col] *= q;
     for (int ps = 0; PS && ps < a.nPs; ps++) {  // point sources: derivatives after the convolution
       const CompF32 &c = a.comps[b * a.nComp + a.psComp[ps]];
       const CompDesc &d = a.desc[a.psComp[ps]];
@@ -1734,6 +1807,7 @@ __global__ void __launch_bounds__(1024) k_fast_jtwj_rows(FastArgs a, FastGeom g,
     }
   }
   __syncthreads();
+  pdl_trigger();
   const int Q = nP * (nP + 1) / 2 + nP + 1;
   float2 *out = part + (long)b * Q * a.partStride + blockIdx.x;
   if (a.count)
@@ -1746,6 +1820,7 @@ __global__ void __launch_bounds__(1024) k_fast_jtwj_rows(FastArgs a, FastGeom g,
 __global__ void __launch_bounds__(256) k_fast_jtwj_reduce(FastArgs a, const float2 *__restrict__ part, int nRows,
                                                          double *__restrict__ alpha, double *__restrict__ beta,
                                                          double *__restrict__ stat) {
+  pdl_wait();
   const int qi = blockIdx.x, b = blockIdx.y, nP = a.nParams;
   const int nPair = nP * (nP + 1) / 2, Q = nPair + nP + 1;
   const float2 *p = part + ((long)b * Q + qi) * a.partStride;
@@ -2106,58 +2181,74 @@ static cudaError_t launch_deriv(const FastArgs &a, const WinDesc &w, const FFTLe
                                 const JtwjArgs &J, cudaStream_t st) {
   const int M = L.half.n;
   const size_t sm = deriv_smem(M, J.nD);
-  k_fast_deriv_r2c<<<dim3(w.rows, nBatch), kJtwjThreads, sm, st>>>(
-      a, w, plan32(L, true), reinterpret_cast<const cplx<float> *>(L.twL32), J.slot, J.nD, win);
-  return cudaGetLastError();
+  return launch_pdl(k_fast_deriv_r2c, dim3(w.rows, nBatch), dim3(kJtwjThreads), sm, st, a, w, plan32(L, true),
+                    reinterpret_cast<const cplx<float> *>(L.twL32), J.slot, J.nD, win);
 }
 
-// Statistic, JtJ and Jt dev of the deviates for nBatch parameter vectors:
-// the forward pass (which leaves the FP32 model image in a.modelOut), the
-// derivative images of every non-background parameter convolved with the PSF
-// (region derivatives through the oversampled pipeline and the block
-// average), then the per-row products and their FP64 sums.
+// Statistic, JtJ and Jt dev of the deviates for nBatch parameter vectors: the
+// set-up and the subsample tables, the derivative images of every
+// non-background parameter convolved with the PSF, then the per-row products
+// (which form the model image from the derivative images) and their FP64
+// sums.  The region's derivative images -- the oversampled pipeline and the
+// block average -- run on the side stream beside the main window's, forked
+// after the set-up and joined before the products.
 cudaError_t fast_jtwj(const FastPlan &p, const FastArgs &a, const JtwjArgs &J, int nBatch, cudaStream_t st) {
   const FastGeom &g = p.g;
-  cudaError_t e = fast_forward(p, a, nBatch, false, st);
-  if (e) return e;
+  if (p.timer) p.timer->n = 0;
+  if (p.timer && !p.timer->only) stage_end(p, "start", st);
   const int nD = J.nD, nB = nBatch * nD;
   const FastTune &tu = p.tune;
+  const WinDesc mw = main_win(g, J.dspec), rw = region_win(g, J.drspec);
+  const bool region = g.hasRegion && nD > 0, fork = region && p.side;
+  cudaStream_t rs = fork ? p.side : st;
+  if (g.hasRegion) {
+    STAGE("setup", st, launch_setup(a, mw, rw, true, nBatch, st));
+  } else {
+    STAGE("setup_subsample", st, launch_setup_subsample(a, mw, rw, false, nBatch, st));
+  }
+  if (fork) {
+    cudaError_t e = cudaEventRecord(p.fork0, st);
+    if (!e) e = cudaStreamWaitEvent(rs, p.fork0, 0);
+    if (e) return e;
+  }
+  if (region) {
+    const float rscale = 1.f / ((float)p.Rx->L * (float)p.Ry->L);
+    STAGE("region_subsample", rs, launch_region_sub(a, rw, nBatch, rs));
+    STAGE("jtwj_region_deriv_r2c", rs, launch_deriv(a, rw, *p.Rx, nBatch, 1, J, rs));
+    STAGE("jtwj_region_cols", rs,
+          launch_cols32(J.drspec, g.rSpecPitch, g.rSpecBatch, p.Rx->L / 2 + 1, g.rWinRows, g.rSubRows, p.Hr,
+                             p.hrPitch, *p.Ry, rscale, 1, nB, rs, tu.colCpb, 0, 1, nullptr, tu.colThreads));
+    const int M = p.Rx->half.n;
+    const size_t sm = sizeof(cplx<float>) * 3 * g.rScale * (M + 1);
+    STAGE("jtwj_region_down", rs,
+          launch_pdl(k_fast_region_down<false>, dim3(g.rRows, nB), dim3(line_threads(M * g.rScale / 2)), sm, rs, a, g,
+                     reinterpret_cast<cplx<float> *>(J.drspec), plan32(*p.Rx, true),
+                     reinterpret_cast<const cplx<float> *>(p.Rx->twL32), J.regDeriv, 0, 0, 0));
+  }
+  if (g.hasRegion) STAGE("subsample", st, launch_subsample(a, mw, nBatch, st));
   if (nD > 0) {
-    if (g.hasRegion) {
-      const float rscale = 1.f / ((float)p.Rx->L * (float)p.Ry->L);
-      STAGE("jtwj_region_deriv_r2c", st, launch_deriv(a, region_win(g, J.drspec), *p.Rx, nBatch, 1, J, st));
-      STAGE("jtwj_region_cols", st,
-            launch_cols32(J.drspec, g.rSpecPitch, g.rSpecBatch, p.Rx->L / 2 + 1, g.rWinRows, g.rSubRows, p.Hr,
-                               p.hrPitch, *p.Ry, rscale, 1, nB, st, tu.colCpb, 0, 1, nullptr, tu.colThreads));
-      const int M = p.Rx->half.n;
-      const size_t sm = sizeof(cplx<float>) * 3 * g.rScale * (M + 1);
-      stage_begin(p, "jtwj_region_down", st);
-      k_fast_region_down<false><<<dim3(g.rRows, nB), line_threads(M * g.rScale / 2), sm, st>>>(
-          a, g, reinterpret_cast<cplx<float> *>(J.drspec), plan32(*p.Rx, true),
-          reinterpret_cast<const cplx<float> *>(p.Rx->twL32), J.regDeriv, 0, 0, 0);
-      if ((e = cudaGetLastError())) return e;
-      stage_end(p, "jtwj_region_down", st);
-    }
     const float scale = 1.f / ((float)p.Lx->L * (float)p.Ly->L);
-    STAGE("jtwj_deriv_r2c", st, launch_deriv(a, main_win(g, J.dspec), *p.Lx, nBatch, 0, J, st));
+    STAGE("jtwj_deriv_r2c", st, launch_deriv(a, mw, *p.Lx, nBatch, 0, J, st));
     STAGE("jtwj_cols", st,
           launch_cols32(J.dspec, g.specPitch, g.specBatch, p.Lx->L / 2 + 1, g.winRows, g.nDataRows, p.H,
                              p.hPitch, *p.Ly, scale, 1, nB, st, tu.colCpb, p.hBatch, nD, p.hMap, tu.colThreads));
   }
+  if (fork) {
+    cudaError_t e = cudaEventRecord(p.join0, rs);
+    if (!e) e = cudaStreamWaitEvent(st, p.join0, 0);
+    if (e) return e;
+  }
   const int M = p.Lx->half.n;
   const size_t sm = jtwj_rows_smem(M, nD, a.nParams, g.nDataCols, kJtwjThreads);
-  stage_begin(p, "jtwj_rows", st);
   auto jrows = a.nPs ? k_fast_jtwj_rows<true> : k_fast_jtwj_rows<false>;
-  jrows<<<dim3(g.nDataRows, nBatch), kJtwjThreads, sm, st>>>(
-      a, g, plan32(*p.Lx, true), reinterpret_cast<const cplx<float> *>(p.Lx->twL32),
-      reinterpret_cast<const cplx<float> *>(J.dspec), J.regDeriv, J.slot, nD, J.part, J.jac);
-  if ((e = cudaGetLastError())) return e;
-  stage_end(p, "jtwj_rows", st);
+  STAGE("jtwj_rows", st,
+        launch_pdl(jrows, dim3(g.nDataRows, nBatch), dim3(kJtwjThreads), sm, st, a, g, plan32(*p.Lx, true),
+                   reinterpret_cast<const cplx<float> *>(p.Lx->twL32), reinterpret_cast<const cplx<float> *>(J.dspec),
+                   J.regDeriv, J.slot, nD, J.part, J.jac));
   const int nP = a.nParams, Q = nP * (nP + 1) / 2 + nP + 1;
-  stage_begin(p, "jtwj_reduce", st);
-  k_fast_jtwj_reduce<<<dim3(Q, nBatch), 256, 0, st>>>(a, J.part, g.nDataRows, J.alpha, J.beta, J.stat);
-  if ((e = cudaGetLastError())) return e;
-  stage_end(p, "jtwj_reduce", st);
+  STAGE("jtwj_reduce", st,
+        launch_pdl(k_fast_jtwj_reduce, dim3(Q, nBatch), dim3(256), 0, st, a, J.part, g.nDataRows, J.alpha, J.beta,
+                   J.stat));
   return cudaSuccess;
 }
 
@@ -2232,79 +2323,6 @@ __global__ void __launch_bounds__(256) k_rag_subsample(FastArgs a, RagArgs r) {
       for (int q = 0; q < 8; q++) dst[q] = acc[q] * dd;
     }
   }
-}
-
-// One window row of one cutout per CTA: evaluated model row, row r2c.
-__global__ void __launch_bounds__(512) k_rag_eval_r2c(FastArgs a, RagArgs r) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  pdl_wait();
-  const int t = blockIdx.x;
-  const int k = rag_slot(r.start, r.K, t);
-  const RagEntry &E = r.ent[r.act[k]];
-  const int row = t - r.start[k];
-  const int M = E.rowPlan.n, ls = M + 1;
-  CompF32 *sc = reinterpret_cast<CompF32 *>(smem);
-  int *boxes = reinterpret_cast<int *>(sc + kMaxComponents);
-  cplx<float> *bufA = reinterpret_cast<cplx<float> *>(boxes + 2 * kMaxComponents);
-  cplx<float> *bufB = bufA + ls;
-  const int nC = a.nComp;
-  for (int i = threadIdx.x; i < nC; i += blockDim.x) {
-    sc[i] = a.comps[k * nC + i];
-    const int *o = a.subBox + ((long)k * nC + i) * 4;
-    boxes[2 * i] = o[0];
-    boxes[2 * i + 1] = o[1];
-  }
-  for (int i = threadIdx.x; i < M; i += blockDim.x) bufA[i] = {0.f, 0.f};
-  __syncthreads();
-  const WinDesc w = rag_win(E, r.spec + E.specOff);
-  const FastDiv byM(M);
-  for (int c = 0; c < nC; c++) {
-    const CompF32 cc = sc[c];
-    if (!in_rows(cc.type)) continue;
-    const float *tab = a.subTab + sub_base(a, k, c, 0);
-    const int bc0 = boxes[2 * c], br0 = boxes[2 * c + 1], side = a.boxMain;
-    const bool box = rows_meet_box(cc, row, 1, br0, side);
-    switch (cc.type) {
-      case F_SERSIC: eval_pixels_rt<F_SERSIC>(false, box, cc, w, row, 1, M, ls, byM, bufA, tab, side, bc0, br0); break;
-      case F_EXP: eval_pixels_rt<F_EXP>(false, box, cc, w, row, 1, M, ls, byM, bufA, tab, side, bc0, br0); break;
-      case F_GRING: eval_pixels_rt<F_GRING>(false, box, cc, w, row, 1, M, ls, byM, bufA, tab, side, bc0, br0); break;
-      case F_MOFFAT: eval_pixels_rt<F_MOFFAT>(false, box, cc, w, row, 1, M, ls, byM, bufA, tab, side, bc0, br0); break;
-      case F_GAUSS: eval_pixels_rt<F_GAUSS>(false, box, cc, w, row, 1, M, ls, byM, bufA, tab, side, bc0, br0); break;
-      case F_TILTEDSKY: eval_pixels_rt<F_TILTEDSKY>(false, box, cc, w, row, 1, M, ls, byM, bufA, tab, side, bc0, br0); break;
-      default: break;
-    }
-  }
-  __syncthreads();
-  cplx<float> *Z = block_fft(bufA, bufB, E.rowPlan, 1, ls, 1, -1, false);
-  pdl_trigger();
-  cplx<float> *out = w.spec + (long)row * E.pitch;
-  for (int kk = threadIdx.x; kk <= M; kk += blockDim.x) out[kk] = r2c_post(Z, kk, M, E.twL);
-}
-
-// One data row of one cutout per CTA: inverse row FFT of the convolved
-// spectrum, the FP32 model row (plus the constant background) to r.model.
-__global__ void __launch_bounds__(512) k_rag_model_rows(FastArgs a, RagArgs r) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  pdl_wait();
-  const int t = blockIdx.x;
-  const int k = rag_slot(r.start, r.K, t);
-  const RagEntry &E = r.ent[r.act[k]];
-  const int row = t - r.start[k];
-  const int M = E.rowPlan.n, ls = M + 1;
-  cplx<float> *bufX = reinterpret_cast<cplx<float> *>(smem);
-  cplx<float> *bufA = bufX + ls;
-  cplx<float> *bufB = bufA + ls;
-  const cplx<float> *in = r.spec + E.specOff + (long)row * E.pitch;
-  for (int kk = threadIdx.x; kk <= M; kk += blockDim.x) bufX[kk] = in[kk];
-  __syncthreads();
-  for (int kk = threadIdx.x; kk < M; kk += blockDim.x) bufA[kk] = c2r_pre(bufX, kk, M, E.twL);
-  __syncthreads();
-  const cplx<float> *Z = block_fft(bufA, bufB, E.rowPlan, 1, ls, 1, +1, false);
-  pdl_trigger();
-  const float *zr = reinterpret_cast<const float *>(Z);
-  const float bg = a.bgLevel[2 * k];
-  float *m = r.model + E.dataOff + (long)row * E.nDataCols;
-  for (int col = threadIdx.x; col < E.nDataCols; col += blockDim.x) m[col] = zr[col] + bg;
 }
 
 // One window row of one cutout per CTA: the nD derivative rows (typed pixel
@@ -2383,6 +2401,7 @@ __global__ void __launch_bounds__(512) k_rag_jtwj_rows(FastArgs a, RagArgs r, co
   cplx<float> *bufA = reinterpret_cast<cplx<float> *>(ss + kMaxParams);
   cplx<float> *bufB = bufA + nD * ls;
   for (int i = threadIdx.x; i < nP; i += blockDim.x) ss[i] = slot[i];
+  find_amplitudes(a, k, slot, ss);
   const cplx<float> *src = r.spec + (long)nD * E.specOff + (long)row * E.pitch;
   const FastDiv byM(M);
   for (int idx = threadIdx.x; idx < nD * M; idx += blockDim.x) {
@@ -2401,7 +2420,7 @@ __global__ void __launch_bounds__(512) k_rag_jtwj_rows(FastArgs a, RagArgs r, co
   float *qb = aux, *dv = qb + 2 * nc, *zero = dv + nc, *red = zero + nc;
   for (int col = threadIdx.x; col < nc; col += blockDim.x) {
     const long z = E.dataOff + (long)row * nc + col;
-    const float m = r.model[z];
+    const float m = model_from_lines(a, k, ss, Zr + col, uStride, a.bgLevel[2 * k]);
     float dev, q;
     deviate_slope(a, z, m, dev, q);
     for (int j = 0; j < nD; j++) Zr[j * uStride + col] *= q;
@@ -2443,12 +2462,6 @@ __global__ void __launch_bounds__(256) k_rag_jtwj_reduce(FastArgs a, RagArgs r, 
   }
 }
 
-static size_t rag_eval_smem(int maxM) {
-  return sizeof(CompF32) * kMaxComponents + sizeof(int) * 2 * kMaxComponents + sizeof(cplx<float>) * 2 * (maxM + 1) +
-         16;
-}
-
-constexpr int kRagRowThreads = 128;
 constexpr int kRagJtwjThreads = 256;
 
 size_t rag_jtwj_smem(int maxM, int nD, int nP, int maxCols) {
@@ -2459,12 +2472,11 @@ size_t rag_jtwj_smem(int maxM, int nD, int nP, int maxCols) {
   return std::max(deriv, rows);
 }
 
-// The whole ragged J^T W J evaluation: forward model (set-up + subsample,
-// window rows + row FFT, column pass x PSF, inverse rows -> model images),
-// derivative images (window rows, column pass x PSF), the per-row products
-// and their FP64 sums per cutout.  r.spec holds the forward spectra, dspec the
-// derivative spectra; starts/totals are the slots' prefix sums and totals per
-// kind of work.
+// The whole ragged J^T W J evaluation: set-up + subsample tables, derivative
+// images (window rows, column pass x PSF), the per-row products (which form
+// the model from the derivative images) and their FP64 sums per cutout.  dspec
+// holds the derivative spectra; starts/totals are the slots' prefix sums and
+// totals per kind of work.
 cudaError_t rag_jtwj(const FastArgs &a, RagArgs r, cplx<float> *dspec, const int *const starts[kRagWorkKinds],
                      const int totals[kRagWorkKinds], const int *slot, int nD, int maxM, size_t colSmem, int colThreads,
                      int maxCols, double *alpha, double *beta, double *stat, cudaStream_t st) {
@@ -2475,19 +2487,6 @@ cudaError_t rag_jtwj(const FastArgs &a, RagArgs r, cplx<float> *dspec, const int
   const int cap = std::max(1, 8 * 152 / std::max(a.nComp * K, 1));
   const int nSub = std::max(1, std::min((a.boxMain * a.boxMain + 7) / 8, cap));
   if ((e = launch_pdl(k_rag_subsample, dim3(nSub, a.nComp, K), dim3(256), 0, st, a, r))) return e;
-  r.start = starts[kRagWinRows];
-  allow_max_smem((const void *)k_rag_eval_r2c);
-  if ((e = launch_pdl(k_rag_eval_r2c, dim3(totals[kRagWinRows]), dim3(kRagRowThreads), rag_eval_smem(maxM), st, a,
-                      r)))
-    return e;
-  r.start = starts[kRagCols];
-  r.lines = 1;
-  if ((e = launch_rag_cols(r, totals[kRagCols], colSmem, colThreads, st))) return e;
-  r.start = starts[kRagDataRows];
-  allow_max_smem((const void *)k_rag_model_rows);
-  if ((e = launch_pdl(k_rag_model_rows, dim3(totals[kRagDataRows]), dim3(kRagRowThreads),
-                      sizeof(cplx<float>) * 3 * (maxM + 1), st, a, r)))
-    return e;
   const size_t smJ = rag_jtwj_smem(maxM, nD, a.nParams, maxCols);
   RagArgs rd = r;
   rd.spec = dspec;

@@ -406,10 +406,9 @@ struct RagArgs {
   const int *act;          // [K] entry of slot k
   const int *start;        // [K + 1] prefix sums of the launch's work count per slot
   int K;
-  int lines;               // column pass: spectra per entry (1, or nD derivative spectra)
-  cplx<float> *spec;       // spectra (forward: specOff; derivatives: nD * specOff + j * specSize)
+  int lines;               // column pass: spectra per entry (nD derivative spectra)
+  cplx<float> *spec;       // derivative spectra (nD * specOff + j * specSize)
   const cplx<float> *H;    // PSF spectra (hOff)
-  float *model;            // FP32 model images (dataOff)
   float2 *part;            // per-row partials (hi, lo) [Q][totalRows] (rowOff)
   long totalRows;
 };
@@ -428,7 +427,7 @@ __device__ __forceinline__ int rag_slot(const int *start, int K, int t) {
 }
 
 // work counts per slot of each ragged stage
-enum RagWork { kRagWinRows = 0, kRagDataRows = 1, kRagCols = 2, kRagDerivCols = 3, kRagWorkKinds = 4 };
+enum RagWork { kRagWinRows = 0, kRagDataRows = 1, kRagDerivCols = 2, kRagWorkKinds = 3 };
 
 cudaError_t rag_jtwj(const FastArgs &a, RagArgs r, cplx<float> *dspec, const int *const starts[kRagWorkKinds],
                      const int totals[kRagWorkKinds], const int *slot, int nD, int maxM, size_t colSmem, int colThreads,

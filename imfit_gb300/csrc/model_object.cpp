@@ -302,7 +302,7 @@ struct imfit_model_s {
   bool fastReady = false;
   FastGeom fg{};
   FFTLen Fx, Fy, FRx, FRy;
-  DevBuf<float> dH32, dHr32, dData32, dW32, dExtra32, dCount32, dBg, dModelOut;
+  DevBuf<float> dH32, dHr32, dData32, dW32, dExtra32, dCount32, dBg;
   DevBuf<float> dCountBatch;  // batched bootstrap: [sample][data pixel] multiplicities
   int bootBatch = 0;          // number of samples while a batched bootstrap fit runs
   DevBuf<float> dSpec32, dRSpec32;  // complex
@@ -352,7 +352,7 @@ struct imfit_model_s {
     }
   } rag;
   DevBuf<RagEntry> dRagEnt;
-  DevBuf<float> dRagData, dRagW, dRagH, dRagModel, dRagPart, dRagSpec, dRagDSpec, dRagBg, dRagSubTab;
+  DevBuf<float> dRagData, dRagW, dRagH, dRagPart, dRagDSpec, dRagBg, dRagSubTab;
   DevBuf<CompF32> dRagComps;
   DevBuf<int> dRagSubBox, dRagWork, dRagSlot;
   DevBuf<double> dRagParams, dRagS, dRagA, dRagB;
@@ -1957,8 +1957,8 @@ struct imfit_model_s {
     if (B <= jtwjCap) return 0;
     const FastGeom &g = fg;
     const int nP = nParamsTot, Q = nP * (nP + 1) / 2 + nP + 1;
-    cudaError_t e = dModelOut.reserve((size_t)B * nDataVals);
-    if (!e && nDeriv) e = dDSpec32.reserve(2 * (size_t)B * nDeriv * g.specBatch);
+    cudaError_t e = cudaSuccess;
+    if (nDeriv) e = dDSpec32.reserve(2 * (size_t)B * nDeriv * g.specBatch);
     if (!e && nDeriv && g.hasRegion) e = dDRSpec32.reserve(2 * (size_t)B * nDeriv * g.rSpecBatch);
     if (!e && nDeriv && g.hasRegion) e = dRegDeriv.reserve((size_t)B * nDeriv * g.rRows * g.rCols);
     if (!e) e = dJPart.reserve(2 * (size_t)B * Q * partStride());  // (hi, lo) pairs
@@ -1989,7 +1989,7 @@ struct imfit_model_s {
     // after the autotuner: its choice of FFT plan sets the derivative spectra's size
     st = ensureJtwjCap(B);
     if (st) return st;
-    FastArgs a = fastArgs(dP, dS, dGrad.p, dModelOut.p);
+    FastArgs a = fastArgs(dP, dS, dGrad.p, nullptr);
     FastPlan p = fastPlan();
     int optin = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
@@ -2225,9 +2225,7 @@ struct imfit_model_s {
     if (!e) e = cudaMemcpy(dRagSlot.p, hRagSlot.data(), sizeof(int) * nParamsTot, cudaMemcpyHostToDevice);
     // evaluation buffers, sized for all cutouts active
     const int nP = nParamsTot, nC = (int)funcs.size(), Q = nP * (nP + 1) / 2 + nP + 1;
-    if (!e) e = dRagSpec.reserve(2 * (size_t)R.totalSpec);
     if (!e && ragNDeriv) e = dRagDSpec.reserve(2 * (size_t)ragNDeriv * R.totalSpec);
-    if (!e) e = dRagModel.reserve(R.totalPix);
     if (!e) e = dRagPart.reserve(2 * (size_t)Q * R.totalRows);  // (hi, lo) pairs
     if (!e) e = dRagParams.reserve((size_t)nImg * nP);
     if (!e) e = dRagS.reserve(nImg);
@@ -2269,7 +2267,6 @@ struct imfit_model_s {
       const RagEntry &E = R.ent[en];
       pre[kRagWinRows][k + 1] = pre[kRagWinRows][k] + E.winRows;
       pre[kRagDataRows][k + 1] = pre[kRagDataRows][k] + E.nDataRows;
-      pre[kRagCols][k + 1] = pre[kRagCols][k] + E.colGroups;
       pre[kRagDerivCols][k + 1] = pre[kRagDerivCols][k] + E.colGroups * ragNDeriv;
     }
     cudaError_t e = cudaMemcpyAsync(dRagWork.p, w.data(), sizeof(int) * w.size(), cudaMemcpyHostToDevice, stream);
@@ -2298,9 +2295,8 @@ struct imfit_model_s {
     r.act = dRagWork.p;
     r.K = K;
     r.lines = 1;
-    r.spec = reinterpret_cast<cplx<float> *>(dRagSpec.p);
+    r.spec = reinterpret_cast<cplx<float> *>(dRagDSpec.p);
     r.H = reinterpret_cast<const cplx<float> *>(dRagH.p);
-    r.model = dRagModel.p;
     r.part = reinterpret_cast<float2 *>(dRagPart.p);
     r.totalRows = R.totalRows;
     const int *starts[kRagWorkKinds];
