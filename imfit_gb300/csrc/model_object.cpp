@@ -346,7 +346,6 @@ struct imfit_model_s {
     int maxM = 0, maxCols = 0;
     size_t colSmem = 0;  // launch shape of the column pass
     int colThreads = 0;
-    std::vector<int> work;  // act, then the prefix arrays, uploaded per evaluation
     ~RagSet() {
       for (auto &kv : lens) fftlen_destroy(*kv.second);
     }
@@ -354,8 +353,8 @@ struct imfit_model_s {
   DevBuf<RagEntry> dRagEnt;
   DevBuf<float> dRagData, dRagW, dRagH, dRagPart, dRagDSpec, dRagBg, dRagSubTab;
   DevBuf<CompF32> dRagComps;
-  DevBuf<int> dRagSubBox, dRagWork, dRagSlot;
-  DevBuf<double> dRagParams, dRagS, dRagA, dRagB;
+  DevBuf<int> dRagSubBox, dRagSlot;
+  DevBuf<double> dRagIn, dRagOut;  // parameters and work lists; statistics, J^T J, J^T dev
   DevBuf<CompDesc> dRagDesc;
   int ragNDeriv = 0;
   std::vector<int> hRagSlot;
@@ -385,6 +384,18 @@ struct imfit_model_s {
   int fastCap = 0;
   bool useGraphs = true;
   Captured graph;
+  // the captured J^T W J evaluation and everything its launches were given
+  // (compared byte by byte; padding is zeroed)
+  struct JtwjKey {
+    FastArgs a;
+    JtwjArgs J;
+    FastGeom g;
+    FastTune tune;
+    long nBatch;
+  };
+  cudaGraphExec_t jtwjGraph = nullptr;
+  JtwjKey jtwjKey;
+  bool jtwjKeySet = false;
   StageTimer timer;
   bool timing = false;
   std::string timingStage;           // empty: time every kernel (serially)
@@ -400,7 +411,7 @@ struct imfit_model_s {
     fftlen_destroy(Fy);
     fftlen_destroy(FRx);
     fftlen_destroy(FRy);
-    if (graph.exec) cudaGraphExecDestroy(graph.exec);
+    dropGraph();
     if (timing)
       for (int i = 0; i < StageTimer::kMax; i++) cudaEventDestroy(timer.ev[i]);
     if (hPinned) cudaFreeHost(hPinned);
@@ -1429,10 +1440,7 @@ struct imfit_model_s {
     jtwjCap = 0;
     fastCap = 0;
     tuned.clear();
-    if (graph.exec) {
-      cudaGraphExecDestroy(graph.exec);
-      graph = Captured{};
-    }
+    dropGraph();
     fastReady = true;
     return 0;
   }
@@ -1515,10 +1523,7 @@ struct imfit_model_s {
     }
     if (e) return cuda_fail(e, "fast batch buffers");
     fastCap = B;
-    if (graph.exec) {
-      cudaGraphExecDestroy(graph.exec);
-      graph = Captured{};
-    }
+    dropGraph();
     return 0;
   }
 
@@ -1562,7 +1567,8 @@ struct imfit_model_s {
 
   FastArgs fastArgs(const double *dP, double *dS, double *dG, float *modelOut) {
     syncPointSourceState();
-    FastArgs a{};
+    FastArgs a;
+    memset(static_cast<void *>(&a), 0, sizeof a);  // the padding too: arguments are compared as bytes
     a.subTab = dSubTab.p;
     a.subBox = dSubBox.p;
     a.boxMain = kBoxMain;
@@ -1909,6 +1915,24 @@ struct imfit_model_s {
     return 0;
   }
 
+  // at least n doubles of page-locked memory that the kernels read and write
+  // directly (hMapped on the host, dMapped on the device)
+  bool mapped(size_t n) {
+    if (n <= hMappedN) return true;
+    if (hMapped) cudaFreeHost(hMapped);
+    hMapped = dMapped = nullptr;
+    hMappedN = 0;
+    if (cudaHostAlloc(&hMapped, sizeof(double) * n, cudaHostAllocMapped) == cudaSuccess &&
+        cudaHostGetDevicePointer(&dMapped, hMapped, 0) == cudaSuccess) {
+      hMappedN = n;
+      return true;
+    }
+    if (hMapped) cudaFreeHost(hMapped);
+    hMapped = dMapped = nullptr;
+    cudaGetLastError();
+    return false;
+  }
+
   int fastHost(int B, const double *params, double *stats, double *grads) {
     int st = prepareFast();
     if (st) return st;
@@ -1916,20 +1940,7 @@ struct imfit_model_s {
     if (st) return st;
     const int nP = nParamsTot;
     const size_t need = (size_t)B * (2 * nP + 1);
-    if (need > hMappedN) {
-      if (hMapped) cudaFreeHost(hMapped);
-      hMapped = dMapped = nullptr;
-      hMappedN = 0;
-      if (cudaHostAlloc(&hMapped, sizeof(double) * need, cudaHostAllocMapped) == cudaSuccess &&
-          cudaHostGetDevicePointer(&dMapped, hMapped, 0) == cudaSuccess) {
-        hMappedN = need;
-      } else {
-        if (hMapped) cudaFreeHost(hMapped);
-        hMapped = dMapped = nullptr;
-        cudaGetLastError();
-      }
-    }
-    if (hMappedN) {  // zero-copy form
+    if (mapped(need)) {  // zero-copy form
       double *hp = hMapped, *hs = hMapped + (size_t)B * nP, *hg = hs + B;
       std::copy(params, params + (size_t)B * nP, hp);
       double *dp = dMapped, *ds = dMapped + (size_t)B * nP, *dg = ds + B;
@@ -1995,7 +2006,8 @@ struct imfit_model_s {
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     if (fast_jtwj_smem(p, nDeriv, nParamsTot) > (size_t)optin)
       return fail(IMFIT_E_UNSUPPORTED, "J^T J: too many parameters for this image width (shared memory)");
-    JtwjArgs J{};
+    JtwjArgs J;
+    memset(static_cast<void *>(&J), 0, sizeof J);
     J.dspec = dDSpec32.p;
     J.drspec = dDRSpec32.p;
     J.regDeriv = dRegDeriv.p;
@@ -2006,11 +2018,50 @@ struct imfit_model_s {
     J.beta = dBt;
     J.stat = dS;
     J.jac = jacOut;
-    cudaError_t e = fast_jtwj(p, a, J, B, stream);
+    cudaError_t e;
+    if (useGraphs && !timing && !jacOut) {
+      // a Levenberg-Marquardt fit repeats the evaluation with the same
+      // arguments: from the second such call on it is captured and replayed
+      // (the lockstep batch, whose size changes from round to round, is not)
+      JtwjKey key;
+      memset(static_cast<void *>(&key), 0, sizeof key);
+      memcpy(static_cast<void *>(&key.a), &a, sizeof a);
+      memcpy(static_cast<void *>(&key.J), &J, sizeof J);
+      memcpy(static_cast<void *>(&key.g), &p.g, sizeof p.g);
+      key.tune = p.tune;
+      key.nBatch = B;
+      const bool same = jtwjKeySet && memcmp(&key, &jtwjKey, sizeof key) == 0;
+      if (!same) {
+        if (jtwjGraph) cudaGraphExecDestroy(jtwjGraph);
+        jtwjGraph = nullptr;
+        memcpy(static_cast<void *>(&jtwjKey), &key, sizeof key);
+        jtwjKeySet = true;
+      } else if (!jtwjGraph) {
+        cudaGraph_t gr;
+        e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
+        if (e) return cuda_fail(e, "graph capture");
+        const cudaError_t e2 = fast_jtwj(p, a, J, B, stream);
+        e = cudaStreamEndCapture(stream, &gr);
+        if (e2) return cuda_fail(e2, "JtWJ launch");
+        if (e) return cuda_fail(e, "graph capture");
+        e = cudaGraphInstantiate(&jtwjGraph, gr, 0);
+        cudaGraphDestroy(gr);
+        if (e) {
+          jtwjGraph = nullptr;
+          return cuda_fail(e, "graph instantiate");
+        }
+      }
+      if (jtwjGraph) {
+        e = cudaGraphLaunch(jtwjGraph, stream);
+        return e ? cuda_fail(e, "graph launch") : 0;
+      }
+    }
+    e = fast_jtwj(p, a, J, B, stream);
     if (e) return cuda_fail(e, "JtWJ launch");
     return 0;
   }
 
+  static constexpr size_t kMappedOut = 16384;  // doubles of results through mapped memory
   // imageMap (host, B entries; image stacks only): batch entry b fits image imageMap[b]
   int jtwjHost(int B, const double *params, double *stats, double *alpha, double *beta,
                const int *imageMap = nullptr) {
@@ -2030,6 +2081,24 @@ struct imfit_model_s {
       curEntry = dEntry.p;
     }
     const int nP = nParamsTot;
+    // one vector or a few: parameters in and results out through mapped
+    // memory, as fastHost (four pageable copies around the kernels took 30 us
+    // of a 203 x 171 evaluation's 134); large batches by copies
+    const size_t nIn = (size_t)B * nP, nOut = (size_t)B * (1 + nP + (size_t)nP * nP);
+    if (nOut <= kMappedOut && mapped(nIn + nOut)) {
+      std::copy(params, params + nIn, hMapped);
+      double *dS = dMapped + nIn, *dA = dS + B, *dBt = dA + (size_t)B * nP * nP;
+      st = enqueueJtwj(B, dMapped, dS, dA, dBt);
+      curEntry = nullptr;
+      if (st) return st;
+      cudaError_t e = cudaStreamSynchronize(stream);
+      if (e) return cuda_fail(e, "JtWJ results");
+      const double *hS = hMapped + nIn, *hA = hS + B, *hB = hA + (size_t)B * nP * nP;
+      std::copy(hS, hS + B, stats);
+      if (alpha) std::copy(hA, hA + (size_t)B * nP * nP, alpha);
+      if (beta) std::copy(hB, hB + nIn, beta);
+      return 0;
+    }
     cudaError_t e = cudaMemcpyAsync(dParams.p, params, sizeof(double) * (size_t)B * nP, cudaMemcpyHostToDevice, stream);
     if (e) return cuda_fail(e, "params upload");
     st = enqueueJtwj(B, dParams.p, dStat.p, dAlpha.p, dBeta.p);
@@ -2227,15 +2296,12 @@ struct imfit_model_s {
     const int nP = nParamsTot, nC = (int)funcs.size(), Q = nP * (nP + 1) / 2 + nP + 1;
     if (!e && ragNDeriv) e = dRagDSpec.reserve(2 * (size_t)ragNDeriv * R.totalSpec);
     if (!e) e = dRagPart.reserve(2 * (size_t)Q * R.totalRows);  // (hi, lo) pairs
-    if (!e) e = dRagParams.reserve((size_t)nImg * nP);
-    if (!e) e = dRagS.reserve(nImg);
-    if (!e) e = dRagA.reserve((size_t)nImg * nP * nP);
-    if (!e) e = dRagB.reserve((size_t)nImg * nP);
+    if (!e) e = dRagIn.reserve((size_t)nImg * nP + (size_t)(kRagWorkKinds + 1) * (nImg + 1));
+    if (!e) e = dRagOut.reserve((size_t)nImg * (1 + nP + (size_t)nP * nP));
     if (!e) e = dRagComps.reserve((size_t)nImg * nC);
     if (!e) e = dRagBg.reserve(2 * (size_t)nImg);
     if (!e) e = dRagSubTab.reserve((size_t)nImg * nC * kBoxMain * kBoxMain * 8);
     if (!e) e = dRagSubBox.reserve((size_t)nImg * nC * 4);
-    if (!e) e = dRagWork.reserve((size_t)(kRagWorkKinds + 1) * (nImg + 1));
     if (e) return cuda_fail(e, "cutout-set buffers");
     int optin = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
@@ -2254,12 +2320,19 @@ struct imfit_model_s {
       return fail(IMFIT_E_ARG, "bad cutout-set J^T J arguments");
     RagSet &R = rag;
     const int nP = nParamsTot;
-    // work lists: act, then per kind the prefix sums of the slots' counts
-    std::vector<int> &w = R.work;
-    w.assign((size_t)(kRagWorkKinds + 1) * (K + 1), 0);
-    int *act = w.data();
+    // one page-locked staging area and one copy each way: the parameters and
+    // the work lists (act, then per kind the prefix sums of the slots' counts)
+    // in, statistics, J^T J and J^T dev out
+    const size_t nIn = (size_t)K * nP, nInts = (size_t)(kRagWorkKinds + 1) * (K + 1), nWork = (nInts + 1) / 2;
+    const size_t nOut = (size_t)K * (1 + nP + (size_t)nP * nP);
+    double *h = pinned(std::max(nIn + nWork, nOut));
+    if (!h) return fail(IMFIT_E_NOMEM, "cutout-set staging");
+    std::copy(params, params + nIn, h);
+    int *w = reinterpret_cast<int *>(h + nIn);
+    memset(w, 0, sizeof(double) * nWork);
+    int *act = w;
     int *pre[kRagWorkKinds];
-    for (int t = 0; t < kRagWorkKinds; t++) pre[t] = w.data() + (size_t)(t + 1) * (K + 1);
+    for (int t = 0; t < kRagWorkKinds; t++) pre[t] = w + (size_t)(t + 1) * (K + 1);
     for (int k = 0; k < K; k++) {
       const int en = entries[k];
       if (en < 0 || en >= R.n) return fail(IMFIT_E_ARG, "cutout index out of range");
@@ -2269,15 +2342,15 @@ struct imfit_model_s {
       pre[kRagDataRows][k + 1] = pre[kRagDataRows][k] + E.nDataRows;
       pre[kRagDerivCols][k + 1] = pre[kRagDerivCols][k] + E.colGroups * ragNDeriv;
     }
-    cudaError_t e = cudaMemcpyAsync(dRagWork.p, w.data(), sizeof(int) * w.size(), cudaMemcpyHostToDevice, stream);
-    if (!e)
-      e = cudaMemcpyAsync(dRagParams.p, params, sizeof(double) * (size_t)K * nP, cudaMemcpyHostToDevice, stream);
+    cudaError_t e = cudaMemcpyAsync(dRagIn.p, h, sizeof(double) * (nIn + nWork), cudaMemcpyHostToDevice, stream);
     if (e) return cuda_fail(e, "cutout-set upload");
+    const int *dWork = reinterpret_cast<const int *>(dRagIn.p + nIn);
+    double *dS = dRagOut.p, *dA = dS + K, *dBt = dA + (size_t)K * nP * nP;
     FastArgs a{};
     a.desc = dRagDesc.p;
     a.nComp = (int)funcs.size();
     a.nParams = nP;
-    a.params = dRagParams.p;
+    a.params = dRagIn.p;
     a.comps = dRagComps.p;
     a.bgLevel = dRagBg.p;
     a.data = dRagData.p;
@@ -2292,7 +2365,7 @@ struct imfit_model_s {
     a.boxReg = 0;
     RagArgs r{};
     r.ent = dRagEnt.p;
-    r.act = dRagWork.p;
+    r.act = dWork;
     r.K = K;
     r.lines = 1;
     r.spec = reinterpret_cast<cplx<float> *>(dRagDSpec.p);
@@ -2302,18 +2375,19 @@ struct imfit_model_s {
     const int *starts[kRagWorkKinds];
     int totals[kRagWorkKinds];
     for (int t = 0; t < kRagWorkKinds; t++) {
-      starts[t] = dRagWork.p + (size_t)(t + 1) * (K + 1);
+      starts[t] = dWork + (size_t)(t + 1) * (K + 1);
       totals[t] = pre[t][K];
     }
     r.start = starts[kRagWinRows];
     e = rag_jtwj(a, r, reinterpret_cast<cplx<float> *>(dRagDSpec.p), starts, totals, dRagSlot.p, ragNDeriv, R.maxM,
-                 R.colSmem, R.colThreads, R.maxCols, dRagA.p, dRagB.p, dRagS.p, stream);
+                 R.colSmem, R.colThreads, R.maxCols, dA, dBt, dS, stream);
     if (e) return cuda_fail(e, "cutout-set J^T J launch");
-    e = cudaMemcpyAsync(stats, dRagS.p, sizeof(double) * K, cudaMemcpyDeviceToHost, stream);
-    if (!e) e = cudaMemcpyAsync(alpha, dRagA.p, sizeof(double) * (size_t)K * nP * nP, cudaMemcpyDeviceToHost, stream);
-    if (!e) e = cudaMemcpyAsync(beta, dRagB.p, sizeof(double) * (size_t)K * nP, cudaMemcpyDeviceToHost, stream);
+    e = cudaMemcpyAsync(h, dRagOut.p, sizeof(double) * nOut, cudaMemcpyDeviceToHost, stream);
     if (!e) e = cudaStreamSynchronize(stream);
     if (e) return cuda_fail(e, "cutout-set J^T J results");
+    std::copy(h, h + K, stats);
+    std::copy(h + K, h + K + (size_t)K * nP * nP, alpha);
+    std::copy(h + K + (size_t)K * nP * nP, h + nOut, beta);
     return 0;
   }
 
@@ -2483,9 +2557,13 @@ struct imfit_model_s {
     return st;
   }
 
+  // both captured evaluations
   void dropGraph() {
     if (graph.exec) cudaGraphExecDestroy(graph.exec);
     graph = Captured{};
+    if (jtwjGraph) cudaGraphExecDestroy(jtwjGraph);
+    jtwjGraph = nullptr;
+    jtwjKeySet = false;
   }
 
   int makeBootstrapSample() {
@@ -3090,20 +3168,14 @@ int imfit_SetKernelTiming(imfit_model_t m, int enable) {
   }
   m->timer.n = 0;
   m->timing = on;
-  if (m->graph.exec) {
-    cudaGraphExecDestroy(m->graph.exec);
-    m->graph = Captured{};
-  }
+  m->dropGraph();
   return 0;
 }
 
 int imfit_SetKernelTimingStage(imfit_model_t m, const char *stage) {
   GET(m);
   m->timingStage = stage ? stage : "";
-  if (m->graph.exec) {
-    cudaGraphExecDestroy(m->graph.exec);
-    m->graph = Captured{};
-  }
+  m->dropGraph();
   return 0;
 }
 
@@ -3111,10 +3183,7 @@ int imfit_SetAutotune(imfit_model_t m, int enable) {
   GET(m);
   m->autotune = enable != 0;
   m->tuned.clear();
-  if (m->graph.exec) {
-    cudaGraphExecDestroy(m->graph.exec);
-    m->graph = Captured{};
-  }
+  m->dropGraph();
   return 0;
 }
 
@@ -3130,10 +3199,7 @@ int imfit_SetLaunchShape(imfit_model_t m, int rowRpb, int rowThreads, int colCpb
     m->hasFixedTune = true;
   }
   m->tuned.clear();
-  if (m->graph.exec) {
-    cudaGraphExecDestroy(m->graph.exec);
-    m->graph = Captured{};
-  }
+  m->dropGraph();
   return 0;
 }
 
@@ -3151,10 +3217,7 @@ int imfit_SetFFTPlan(imfit_model_t m, int candidate, int radixOrder) {
   }
   m->fastReady = false;
   m->tuned.clear();
-  if (m->graph.exec) {
-    cudaGraphExecDestroy(m->graph.exec);
-    m->graph = Captured{};
-  }
+  m->dropGraph();
   return 0;
 }
 
@@ -3189,10 +3252,7 @@ int imfit_GetLaunchShape(imfit_model_t m, int *rowRpb, int *rowThreads, int *col
 int imfit_SetConcurrentRegions(imfit_model_t m, int enable) {
   GET(m);
   m->concurrent = enable != 0;
-  if (m->graph.exec) {
-    cudaGraphExecDestroy(m->graph.exec);
-    m->graph = Captured{};
-  }
+  m->dropGraph();
   return 0;
 }
 
