@@ -1266,7 +1266,7 @@ __device__ __forceinline__ void los_pixel(const WinDesc &w, const CompF32 &cc, i
   yp = fmaf(-dx, cc.sinPA, dy * cc.cosPA);
 }
 
-// Kept partitions: [B][nLos][window pixels][32] panels (lo, hi) and the panel
+// Kept partitions: [B][nLos][32][window pixels] panels (lo, hi) and the panel
 // counts, so the gradient pass integrates the derivatives over the forward
 // pass's panels instead of searching again.
 struct LosStore {
@@ -1282,81 +1282,171 @@ __device__ __forceinline__ int los_index(const CompF32 *sc, int c) {
   return k;
 }
 
-// One warp per window pixel (grid-stride): sum of the 3-D components' line of
-// sight integrals, written to w.losVal (added to the model row by eval_r2c);
-// with a store, each partition is kept for the gradient pass.
-__global__ void __launch_bounds__(256) k_fast_los_eval(FastArgs a, WinDesc w, LosStore ks) {
+// A warp takes runs of 32 adjacent pixels; the warps of a CTA are far apart in
+// the image, so that every SM gets the same mix of cheap and costly pixels.
+// The loops are uniform over the warp: first pixel of a run, stride.
+__device__ __forceinline__ long los_first() { return ((long)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32; }
+__device__ __forceinline__ long los_stride() { return (long)gridDim.x * blockDim.x; }
+
+// Value of component c at this lane's pixel (valid: it exists); with panels,
+// the partition is kept: panel i at panels[i * npix], the number in *count.
+// Bound by the SFU and FP32 pipes: 4 transcendentals and about 25 instructions
+// a node.
+template <bool DISK>
+__device__ __forceinline__ float los_pixel_value(const CompF32 &c, bool valid, float xp, float yp, float2 *panels,
+                                                 int *count, long npix) {
+  const int lane = threadIdx.x & 31;
+  LosPanels P;
+  float total = 0.f, tol = 0.f;
+  bool more = false;
+  int np = 0;
+  if (valid) {
+    np = los_partition<DISK>(c, xp, yp, P, total, more, tol);
+    if (panels && !more)
+      for (int i = 0; i < np; i++) panels[i * npix] = make_float2(P.lo[i], P.hi[i]);
+  }
+  for (unsigned left = __ballot_sync(0xffffffffu, more); left; left &= left - 1) {
+    const int src = __ffs(left) - 1;
+    float lo, hi, t;
+    const int n = los_finish_warp<DISK>(c, __shfl_sync(0xffffffffu, xp, src), __shfl_sync(0xffffffffu, yp, src), P,
+                                        tol, src, lo, hi, t);
+    // the run's pixels are adjacent: lane src's panels are at its pointer
+    if (panels && lane < n) (panels + (src - lane))[lane * npix] = make_float2(lo, hi);
+    if (lane == src) {
+      total = t;
+      np = n;
+    }
+  }
+  if (panels && valid) *count = np;
+  return total;
+}
+
+// Sum of the 3-D components' line of sight integrals of every window pixel,
+// written to w.losVal (added to the model row by eval_r2c).
+__global__ void __launch_bounds__(256, 4) k_fast_los_eval(FastArgs a, WinDesc w, LosStore ks) {
   pdl_wait();
   __shared__ CompF32 sc[kMaxComponents];
   const int b = blockIdx.y;
-  const int nC = a.nComp;
+  const int nC = a.nComp, lane = threadIdx.x & 31;
   for (int i = threadIdx.x; i < nC; i += blockDim.x) sc[i] = a.comps[b * nC + i];
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const GkLane nd = gk21_lane();
   const long npix = (long)w.rows * w.cols;
-  const long nWarps = (long)gridDim.x * (blockDim.x >> 5);
-  for (long p = blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5); p < npix; p += nWarps) {
+  for (long p0 = los_first(); p0 < npix; p0 += los_stride()) {
+    const long p = p0 + lane;
+    const bool valid = p < npix;
     const int row = (int)(p / w.cols), col = (int)(p - (long)row * w.cols);
     float v = 0.f;
     for (int c = 0; c < nC; c++) {
-      const CompF32 &cc = sc[c];
+      const CompF32 cc = sc[c];
       if (!is_los(cc.type)) continue;
       float xp, yp;
       los_pixel(w, cc, row, col, xp, yp);
-      float lo, hi, total;
-      const int np = los_partition(cc, xp, yp, nd, lo, hi, total);
-      v += total;
-      if (ks.panels) {
-        const long slot = ((long)b * ks.nLos + los_index(sc, c)) * npix + p;
-        if (lane < np) ks.panels[slot * 32 + lane] = make_float2(lo, hi);
-        if (lane == 0) ks.count[slot] = np;
-      }
+      const long slot = (long)b * ks.nLos + los_index(sc, c);
+      float2 *pan = ks.panels ? ks.panels + slot * kLosMaxPanels * npix + p : nullptr;
+      int *cnt = ks.panels ? ks.count + slot * npix + p : nullptr;
+      v += cc.type == F_EXPDISK3D ? los_pixel_value<true>(cc, valid, xp, yp, pan, cnt, npix)
+                                  : los_pixel_value<false>(cc, valid, xp, yp, pan, cnt, npix);
     }
-    if (lane == 0) w.losVal[(long)b * npix + p] = v;
+    if (valid) w.losVal[(long)b * npix + p] = v;
   }
 }
 
-// One warp per window pixel: r~ * d(line-of-sight value)/d(parameters) of
-// every 3-D component, per-warp rows in shared memory (no atomics), then one
-// FP32 partial per parameter for this CTA.
-// four CTAs per SM (64 registers): the measured optimum for the gradient pass
+// r~ * d(line-of-sight value)/d(parameters) of component c over this warp's
+// pixels, added to the lanes' sums acc.  The sum runs over pixels and panels
+// alike, so with kept partitions a run's (pixel, panel) pairs are dealt to the
+// lanes evenly: lane t takes pairs t, t + 32, ... of the run's list, found in
+// the prefix sums of the panel counts.
+template <bool DISK>
+__device__ __forceinline__ void los_grad_pixels(const WinDesc &w, const CompF32 &cc, const float *rt,
+                                                const float2 *panels, const int *count, long npix, float *acc) {
+  const int lane = threadIdx.x & 31;
+  for (long p0 = los_first(); p0 < npix; p0 += los_stride()) {
+    const long p = p0 + lane;
+    const float r = p < npix ? rt[p] : 0.f;
+    const int row = (int)(p / w.cols), col = (int)(p - (long)row * w.cols);
+    float xp, yp;
+    los_pixel(w, cc, row, col, xp, yp);
+    if (panels) {
+      const int np = r != 0.f ? count[p] : 0;
+      int end = np;  // inclusive prefix sum
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= o) end += t;
+      }
+      const int total = __shfl_sync(0xffffffffu, end, 31);
+      for (int t0 = 0; t0 < total; t0 += 32) {
+        const int t = t0 + lane;
+        int src = 0;  // the first lane whose end exceeds t
+        for (int o = 16; o > 0; o >>= 1)
+          if (__shfl_sync(0xffffffffu, end, src + o - 1) <= t) src += o;
+        src = min(src, 31);
+        const int i = t - (__shfl_sync(0xffffffffu, end, src) - __shfl_sync(0xffffffffu, np, src));
+        const float sx = __shfl_sync(0xffffffffu, xp, src), sy = __shfl_sync(0xffffffffu, yp, src);
+        const float sr = __shfl_sync(0xffffffffu, r, src);
+        if (t < total) {
+          const float2 pn = panels[i * npix + p0 + src];
+          los_grad_panel<DISK>(cc, sx, sy, pn.x, pn.y, sr, acc);
+        }
+      }
+    } else {
+      LosPanels P;
+      float total, tol = 0.f;
+      bool more = false;
+      if (r != 0.f) {
+        const int np = los_partition<DISK>(cc, xp, yp, P, total, more, tol);
+        if (!more)
+          for (int i = 0; i < np; i++) los_grad_panel<DISK>(cc, xp, yp, P.lo[i], P.hi[i], r, acc);
+      }
+      for (unsigned left = __ballot_sync(0xffffffffu, more); left; left &= left - 1) {
+        const int src = __ffs(left) - 1;
+        const float sx = __shfl_sync(0xffffffffu, xp, src), sy = __shfl_sync(0xffffffffu, yp, src);
+        const float sr = __shfl_sync(0xffffffffu, r, src);
+        float lo, hi;
+        const int n = los_finish_warp<DISK>(cc, sx, sy, P, tol, src, lo, hi, total);
+        if (lane < n) los_grad_panel<DISK>(cc, sx, sy, lo, hi, sr, acc);
+      }
+    }
+  }
+}
+
+// The gradient terms of every 3-D component: FP32 sums per thread and warp,
+// double-float across the warps, one partial per parameter for this CTA.
+// The components are one loop over the pixels each, so that the sums of one
+// stay in registers.
 __global__ void __launch_bounds__(256, 4) k_fast_los_grad(FastArgs a, WinDesc w, float2 *__restrict__ gradPart,
                                                       int blockBase, LosStore ks, int doneTotal) {
   pdl_wait();
   __shared__ CompF32 sc[kMaxComponents];
-  __shared__ float red[8][kMaxParams];
+  __shared__ ffloat red[8][kMaxParams];
   const int b = blockIdx.y;
   const int nC = a.nComp, nP = a.nParams;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int i = threadIdx.x; i < nC; i += blockDim.x) sc[i] = a.comps[b * nC + i];
-  for (int i = threadIdx.x; i < 8 * kMaxParams; i += blockDim.x) (&red[0][0])[i] = 0.f;
+  for (int i = threadIdx.x; i < 8 * kMaxParams; i += blockDim.x) (&red[0][0])[i] = ffloat{0.f, 0.f};
   __syncthreads();
-  const GkLane nd = gk21_lane();
   const long npix = (long)w.rows * w.cols;
-  const long nWarps = (long)gridDim.x * (blockDim.x >> 5);
-  for (long p = blockIdx.x * (long)(blockDim.x >> 5) + wid; p < npix; p += nWarps) {
-    const float r = w.losRt[(long)b * npix + p];
-    if (r == 0.f) continue;
-    const int row = (int)(p / w.cols), col = (int)(p - (long)row * w.cols);
-    for (int c = 0; c < nC; c++) {
-      const CompF32 &cc = sc[c];
-      if (!is_los(cc.type)) continue;
-      float xp, yp, g[kLosGrad];
-      los_pixel(w, cc, row, col, xp, yp);
-      if (ks.panels) {
-        const long slot = ((long)b * ks.nLos + los_index(sc, c)) * npix + p;
-        const int np = ks.count[slot];
-        const float2 pn = lane < np ? ks.panels[slot * 32 + lane] : make_float2(0.f, 0.f);
-        los_grad_panels(cc, xp, yp, nd, np, pn.x, pn.y, g);
-      } else {
-        los_grad_warp(cc, xp, yp, nd, g);
-      }
-      if (lane == 0) {
-        red[wid][cc.x0Index] += r * g[0];
-        red[wid][cc.x0Index + 1] += r * g[1];
-        const int npf = los_nparams(cc);
-        for (int q = 0; q < npf; q++) red[wid][cc.paramOffset + q] += r * g[2 + q];
+  const float *rt = w.losRt + (long)b * npix;
+  for (int c = 0; c < nC; c++) {
+    const CompF32 cc = sc[c];
+    if (!is_los(cc.type)) continue;
+    float acc[kLosGrad];
+#pragma unroll
+    for (int q = 0; q < kLosGrad; q++) acc[q] = 0.f;
+    const long slot = (long)b * ks.nLos + los_index(sc, c);
+    const float2 *pan = ks.panels ? ks.panels + slot * kLosMaxPanels * npix : nullptr;
+    const int *cnt = ks.panels ? ks.count + slot * npix : nullptr;
+    if (cc.type == F_EXPDISK3D)
+      los_grad_pixels<true>(w, cc, rt, pan, cnt, npix, acc);
+    else
+      los_grad_pixels<false>(w, cc, rt, pan, cnt, npix, acc);
+#pragma unroll
+    for (int q = 0; q < kLosGrad; q++) acc[q] = warp_sum(acc[q]);
+    if (lane == 0) {
+      const int npf = los_nparams(cc);
+#pragma unroll
+      for (int q = 0; q < kLosGrad; q++) {
+        const int j = q < 2 ? cc.x0Index + q : (q - 2 < npf ? cc.paramOffset + q - 2 : -1);
+        if (j >= 0) red[wid][j] = ff_add(red[wid][j], acc[q]);
       }
     }
   }

@@ -300,7 +300,7 @@ struct FastArgs {
   // region window, [B][rows][cols] each (all null otherwise)
   float *losVal, *losRt, *rLosVal, *rLosRt;
   // their line-of-sight partitions kept from the forward pass for the gradient
-  // pass ([B][nLos][window pixels][32] (lo, hi) pairs and counts), or null
+  // pass ([B][nLos][32][window pixels] (lo, hi) pairs and counts), or null
   float *losPan, *rLosPan;
   int *losCnt, *rLosCnt;
   int nLos;
