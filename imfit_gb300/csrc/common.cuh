@@ -766,6 +766,98 @@ __device__ __forceinline__ int radial_grad_t(const CompF32 &c, const Geo &g, flo
   return np;
 }
 
+// Sums over pixels of r times the derivatives of radial_grad_t, with the
+// factors that are the same for every pixel of a component taken out of the
+// loop: about 30 instructions a pixel instead of 65 (Sersic), and fold()
+// applies them once a thread.
+template <int TY>
+struct GradSums {
+  // sums of w xp, w ys, w xp yp, w ys^2, where G = dI/dr / r = (component
+  // factor) w; and of the profile parameters' pixel terms
+  float A = 0.f, B = 0.f, C = 0.f, D = 0.f, p0 = 0.f, p1 = 0.f, p2 = 0.f, p3 = 0.f;
+
+  __device__ __forceinline__ void geometry(float wx, float wy, const Geo &g) {
+    A += wx;
+    B += wy;
+    C = fmaf(wx, g.yp, C);
+    D = fmaf(wy, g.ys, D);
+  }
+
+  __device__ __forceinline__ void add(const CompF32 &c, const Geo &g, float r) {
+    if constexpr (TY == F_SERSIC) {
+      const float rinv = (g.r2 > 0.f) ? rsqrtf(g.r2) : 0.f;
+      const float lr = 0.5f * fast_lg2(g.r2) - c.s2;  // log2(r / r_e)
+      const float u = fast_ex2(lr * c.s3);
+      const float rE = r * fast_ex2(c.s1 - c.s1 * u), rEu = rE * u, w = rEu * rinv;
+      geometry(w * (g.xp * rinv), w * (g.ys * rinv), g);
+      p0 += rE;
+      p1 += rEu;
+      p2 = fmaf(rE, u - 1.f, p2);
+      p3 = fmaf(rEu, (u > 0.f) ? lr : 0.f, p3);
+    } else if constexpr (TY == F_EXP) {
+      const float rinv = (g.r2 > 0.f) ? rsqrtf(g.r2) : 0.f, rad = g.r2 * rinv;
+      const float rE = r * fast_ex2(-rad * c.s1), w = rE * rinv;
+      geometry(w * g.xp, w * g.ys, g);
+      p0 += rE;
+      p1 = fmaf(rE, rad, p1);
+    } else if constexpr (TY == F_GRING) {
+      const float rinv = (g.r2 > 0.f) ? rsqrtf(g.r2) : 0.f, dd = g.r2 * rinv - c.s1;
+      const float rE = r * fast_ex2(-dd * dd * c.s2), rEd = rE * dd, w = rEd * rinv;
+      geometry(w * g.xp, w * g.ys, g);
+      p0 += rE;
+      p1 += rEd;
+      p2 = fmaf(rEd, dd, p2);
+    } else if constexpr (TY == F_MOFFAT) {
+      const float Dq = fmaf(g.r2, c.s1, 1.f), lD = fast_lg2(Dq);
+      const float rE = r * fast_ex2(-c.s2 * lD), w = rE * __fdividef(1.f, Dq);  // Dq >= 1
+      geometry(w * g.xp, w * g.ys, g);
+      p0 += rE;
+      p1 = fmaf(w, g.r2, p1);
+      p2 = fmaf(rE, lD, p2);
+    } else {  // F_GAUSS
+      const float w = r * fast_ex2(-g.r2 * c.s1);
+      geometry(w * g.xp, w * g.ys, g);
+      p0 += w;
+      p1 = fmaf(w, g.r2, p1);
+    }
+  }
+
+  // out: the sums of radial_grad_t's out[] over the pixels added
+  __device__ __forceinline__ void fold(const CompF32 &c, float *out) const {
+    float k;  // G = k w
+    if constexpr (TY == F_SERSIC) {
+      const float t = c.s0 * c.s4 * c.s3;
+      k = -t;
+      out[4] = -c.s0 * (c.s5 * p2 - c.s4 * (float)kLn2 * p3 * c.s3 * c.s3);
+      out[5] = p0;
+      out[6] = t * c.pad * p1;
+    } else if constexpr (TY == F_EXP) {
+      k = -c.s0 * c.s3;
+      out[4] = p0;
+      out[5] = c.s0 * c.s3 * c.s3 * p1;
+    } else if constexpr (TY == F_GRING) {
+      k = -c.s0 * c.s4;
+      out[4] = p0;
+      out[5] = c.s0 * c.s4 * p1;
+      out[6] = c.s0 * c.s4 * c.pad * p2;
+    } else if constexpr (TY == F_MOFFAT) {
+      k = -2.f * c.s0 * c.s2 * c.s1;
+      const float alpha = 2.f * c.s0 * c.s2 * c.s1 * c.s6 * p1;
+      out[4] = p0;
+      out[5] = alpha * c.s3 * c.s7;
+      out[6] = -c.s0 * (float)kLn2 * p2 + alpha * c.s5;
+    } else {  // F_GAUSS
+      k = -c.s0 * c.s4;
+      out[4] = p0;
+      out[5] = c.s0 * c.s4 * c.s3 * p1;
+    }
+    out[0] = k * (-c.cosPA * A + c.sinPA * c.invq * B);
+    out[1] = k * (-c.sinPA * A - c.cosPA * c.invq * B);
+    out[2] = k * (float)kDeg2Rad * (1.f - c.invq * c.invq) * C;
+    out[3] = k * c.invq * D;
+  }
+};
+
 // The same with the type chosen at run time.
 __device__ inline int radial_grad32(const CompF32 &c, const Geo &g, float scale, float *out,
                                     float *value = nullptr) {

@@ -68,6 +68,38 @@ __device__ __forceinline__ bool subsampling_type(int t) {
   return t == F_SERSIC || t == F_EXP || t == F_MOFFAT || t == F_GAUSS;
 }
 
+// How the threads of a CTA share nl lines: where the warps divide evenly among
+// the lines, each warp keeps to one line (first line l0, step dl) and strides
+// over its points (first k0, step dk); else all warps take the lines one after
+// the other.  A warp's line index and everything derived from it are then
+// loop constants, and a step along the line costs one addition, where a flat
+// index costs a division (four instructions, two of them on the SFU) and two
+// integer-to-float conversions a point.  256 vectors of a 512 x 512 image,
+// three components, same launch shape (4 lines, 256 threads): eval 531 to 512
+// us; gradient, with GradSums, 1057 to 934 us.
+struct LineWalk {
+  int l0, dl, k0, dk;
+  __device__ __forceinline__ explicit LineWalk(int nl) {
+    const int nw = blockDim.x >> 5, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int wpl = FastDiv(nl).div(nw);  // warps per line
+    if (wpl < 1 || wpl * nl != nw) {
+      wpl = nw;
+      dl = 1;
+    } else {
+      dl = nl;
+    }
+    l0 = FastDiv(wpl).div(wid);
+    k0 = (wid - l0 * wpl) * 32 + lane;
+    dk = wpl * 32;
+  }
+  // f(line, point) for every point of nl lines of n points
+  template <typename F>
+  __device__ __forceinline__ void each(int nl, int n, F f) const {
+    for (int l = l0; l < nl; l += dl)
+      for (int k = k0; k < n; k += dk) f(l, k);
+  }
+};
+
 // Offsets (dx, dy) of window pixel (row, col) from component c's centre,
 // the integer parts exact and the fractions added once.  REG: the window is
 // an oversampled region (fixed at compile time in the pixel loops, so the
@@ -532,53 +564,59 @@ __device__ __forceinline__ float sub_value(const FastArgs &a, const int *box, in
 // ------------------------------------------------------ eval + row r2c
 // Adds component cc's value at every pixel of the CTA's rows to the row
 // buffer (one thread per complex point = two pixels; every pass maps the
-// same points to the same thread, so the passes need no barrier).
+// same points to the same thread, so the passes need no barrier).  On the main
+// window the column offset advances in FP32 (whole numbers: exact).
 template <int TY, bool REG, bool BOX>
-__device__ __forceinline__ void eval_pixels(const CompF32 cc, const WinDesc &w, int row0, int nl, int M, int ls,
-                                            const FastDiv &byM, cplx<float> *buf, const float *tab, int side,
-                                            int bc0, int br0) {
-  for (int idx = threadIdx.x; idx < nl * M; idx += blockDim.x) {
-    const int l = byM.div(idx), k = idx - l * M;
+__device__ __forceinline__ void eval_pixels(const CompF32 cc, const WinDesc &w, const LineWalk &W, int row0, int nl,
+                                            int M, int ls, cplx<float> *buf, const float *tab, int side, int bc0,
+                                            int br0) {
+  for (int l = W.l0; l < nl; l += W.dl) {
     const int row = row0 + l;
-    float v[2] = {0.f, 0.f};
+    float dxf, dyf;
+    win_offsets_t<false>(w, cc, row, 0, dxf, dyf);
+    float xi = (float)(2 * W.k0 + w.xOrig - cc.x0i);
+    const float step = (float)(2 * W.dk);
+    for (int k = W.k0; k < M; k += W.dk, xi += step) {
+      float v[2] = {0.f, 0.f};
 #pragma unroll
-    for (int e = 0; e < 2; e++) {
-      const int col = 2 * k + e;
-      if (col >= w.cols) continue;
-      float dx, dy;
-      win_offsets_t<REG>(w, cc, row, col, dx, dy);
-      if constexpr (TY == F_TILTEDSKY) {
-        v[e] = plane32(cc, dx, dy);
-      } else {
-        const Geo g = geo32(cc, dx, dy);
-        if (BOX && subsampling_t<TY>() && g.r2 < 100.f && n_subsamples32(cc, fast_sqrt(g.r2)) > 1) {
-          // subsampled pixel: the precomputed table (a direct average outside
-          // the box, which the radius bound rules out)
-          const int br = row - br0, bc = col - bc0;
-          v[e] = (br >= 0 && br < side && bc >= 0 && bc < side) ? tab[((long)br * side + bc) * 8]
-                                                                : comp_value32(cc, dx, dy, nullptr);
+      for (int e = 0; e < 2; e++) {
+        const int col = 2 * k + e;
+        if (col >= w.cols) continue;
+        float dx = (xi + (float)e) - cc.x0r, dy = dyf;
+        if constexpr (REG) win_offsets_t<REG>(w, cc, row, col, dx, dy);
+        if constexpr (TY == F_TILTEDSKY) {
+          v[e] = plane32(cc, dx, dy);
         } else {
-          v[e] = radial_t<TY>(cc, g.r2);
+          const Geo g = geo32(cc, dx, dy);
+          if (BOX && subsampling_t<TY>() && g.r2 < 100.f && n_subsamples32(cc, fast_sqrt(g.r2)) > 1) {
+            // subsampled pixel: the precomputed table (a direct average outside
+            // the box, which the radius bound rules out)
+            const int br = row - br0, bc = col - bc0;
+            v[e] = (br >= 0 && br < side && bc >= 0 && bc < side) ? tab[((long)br * side + bc) * 8]
+                                                                  : comp_value32(cc, dx, dy, nullptr);
+          } else {
+            v[e] = radial_t<TY>(cc, g.r2);
+          }
         }
       }
+      cplx<float> &z = buf[l * ls + k];
+      z.x += v[0];
+      z.y += v[1];
     }
-    cplx<float> &z = buf[l * ls + k];
-    z.x += v[0];
-    z.y += v[1];
   }
 }
 
 // eval_pixels with the window kind and the box test chosen at run time
 template <int TY>
-__device__ __forceinline__ void eval_pixels_rt(bool reg, bool box, const CompF32 &cc, const WinDesc &w, int row0,
-                                               int nl, int M, int ls, const FastDiv &byM, cplx<float> *buf,
+__device__ __forceinline__ void eval_pixels_rt(bool reg, bool box, const CompF32 &cc, const WinDesc &w,
+                                               const LineWalk &W, int row0, int nl, int M, int ls, cplx<float> *buf,
                                                const float *tab, int side, int bc0, int br0) {
   if (reg) {
-    if (box) eval_pixels<TY, true, true>(cc, w, row0, nl, M, ls, byM, buf, tab, side, bc0, br0);
-    else eval_pixels<TY, true, false>(cc, w, row0, nl, M, ls, byM, buf, tab, side, bc0, br0);
+    if (box) eval_pixels<TY, true, true>(cc, w, W, row0, nl, M, ls, buf, tab, side, bc0, br0);
+    else eval_pixels<TY, true, false>(cc, w, W, row0, nl, M, ls, buf, tab, side, bc0, br0);
   } else {
-    if (box) eval_pixels<TY, false, true>(cc, w, row0, nl, M, ls, byM, buf, tab, side, bc0, br0);
-    else eval_pixels<TY, false, false>(cc, w, row0, nl, M, ls, byM, buf, tab, side, bc0, br0);
+    if (box) eval_pixels<TY, false, true>(cc, w, W, row0, nl, M, ls, buf, tab, side, bc0, br0);
+    else eval_pixels<TY, false, false>(cc, w, W, row0, nl, M, ls, buf, tab, side, bc0, br0);
   }
 }
 
@@ -603,11 +641,8 @@ __global__ void __launch_bounds__(1024) k_fast_eval_r2c(FastArgs a, WinDesc w, F
   const int nl = min(rpb, w.rows - row0);
   __syncthreads();
   if (nl <= 0) return;
-  const FastDiv byM(M), byM1(M + 1);
-  for (int idx = threadIdx.x; idx < nl * M; idx += blockDim.x) {
-    const int l = byM.div(idx);
-    bufA[l * ls + idx - l * M] = {0.f, 0.f};
-  }
+  const LineWalk W(nl);
+  W.each(nl, M, [&](int l, int k) { bufA[l * ls + k] = {0.f, 0.f}; });
   const int side = win ? a.boxReg : a.boxMain;
   for (int c = 0; c < nC; c++) {
     const CompF32 cc = sc[c];
@@ -616,32 +651,30 @@ __global__ void __launch_bounds__(1024) k_fast_eval_r2c(FastArgs a, WinDesc w, F
     const int bc0 = boxes[2 * c], br0 = boxes[2 * c + 1];
     const bool box = rows_meet_box(cc, row0, nl, br0, side);
     switch (cc.type) {
-      case F_SERSIC: eval_pixels_rt<F_SERSIC>(w.isRegion, box, cc, w, row0, nl, M, ls, byM, bufA, tab, side, bc0, br0); break;
-      case F_EXP: eval_pixels_rt<F_EXP>(w.isRegion, box, cc, w, row0, nl, M, ls, byM, bufA, tab, side, bc0, br0); break;
-      case F_GRING: eval_pixels_rt<F_GRING>(w.isRegion, box, cc, w, row0, nl, M, ls, byM, bufA, tab, side, bc0, br0); break;
-      case F_MOFFAT: eval_pixels_rt<F_MOFFAT>(w.isRegion, box, cc, w, row0, nl, M, ls, byM, bufA, tab, side, bc0, br0); break;
-      case F_GAUSS: eval_pixels_rt<F_GAUSS>(w.isRegion, box, cc, w, row0, nl, M, ls, byM, bufA, tab, side, bc0, br0); break;
-      case F_TILTEDSKY: eval_pixels_rt<F_TILTEDSKY>(w.isRegion, box, cc, w, row0, nl, M, ls, byM, bufA, tab, side, bc0, br0); break;
+      case F_SERSIC: eval_pixels_rt<F_SERSIC>(w.isRegion, box, cc, w, W, row0, nl, M, ls, bufA, tab, side, bc0, br0); break;
+      case F_EXP: eval_pixels_rt<F_EXP>(w.isRegion, box, cc, w, W, row0, nl, M, ls, bufA, tab, side, bc0, br0); break;
+      case F_GRING: eval_pixels_rt<F_GRING>(w.isRegion, box, cc, w, W, row0, nl, M, ls, bufA, tab, side, bc0, br0); break;
+      case F_MOFFAT: eval_pixels_rt<F_MOFFAT>(w.isRegion, box, cc, w, W, row0, nl, M, ls, bufA, tab, side, bc0, br0); break;
+      case F_GAUSS: eval_pixels_rt<F_GAUSS>(w.isRegion, box, cc, w, W, row0, nl, M, ls, bufA, tab, side, bc0, br0); break;
+      case F_TILTEDSKY: eval_pixels_rt<F_TILTEDSKY>(w.isRegion, box, cc, w, W, row0, nl, M, ls, bufA, tab, side, bc0, br0); break;
       default: break;
     }
   }
   if (w.losVal) {  // the 3-D components' line-of-sight sums
-    for (int idx = threadIdx.x; idx < nl * M; idx += blockDim.x) {
-      const int l = byM.div(idx), k = idx - l * M;
+    W.each(nl, M, [&](int l, int k) {
       const float *lv = w.losVal + ((long)b * w.rows + row0 + l) * w.cols;
       cplx<float> &z = bufA[l * ls + k];
       if (2 * k < w.cols) z.x += lv[2 * k];
       if (2 * k + 1 < w.cols) z.y += lv[2 * k + 1];
-    }
+    });
   }
   __syncthreads();
   cplx<float> *Z = block_fft(bufA, bufB, plan, nl, ls, 1, -1, false);
   pdl_trigger();
   cplx<float> *out = w.spec + (long)b * w.specBatch;
-  for (int idx = threadIdx.x; idx < nl * (M + 1); idx += blockDim.x) {
-    const int l = byM1.div(idx), k = idx - l * (M + 1);
+  W.each(nl, M + 1, [&](int l, int k) {
     out[(long)(row0 + l) * w.specPitch + k] = r2c_post(Z + l * ls, k, M, twL);
-  }
+  });
 }
 
 // ------------------------------------------------------------ point sources
@@ -1035,24 +1068,17 @@ __global__ void __launch_bounds__(1024) k_fast_stat_rows(FastArgs a, FastGeom g,
     a.weight += img * a.dataStride;
   }
   if (a.count && a.countStride) a.count += (a.entry ? a.entry[b] : b) * a.countStride;  // batched bootstrap
-  const FastDiv byM(M), byM1(M + 1);
   if (nl > 0) {
-    for (int idx = threadIdx.x; idx < nl * (M + 1); idx += blockDim.x) {
-      const int l = byM1.div(idx), k = idx - l * (M + 1);
-      bufX[l * ls + k] = spec[(long)(row0 + l) * g.specPitch + k];
-    }
+    const LineWalk W(nl);
+    W.each(nl, M + 1, [&](int l, int k) { bufX[l * ls + k] = spec[(long)(row0 + l) * g.specPitch + k]; });
     __syncthreads();
-    for (int idx = threadIdx.x; idx < nl * M; idx += blockDim.x) {
-      const int l = byM.div(idx), k = idx - l * M;
-      bufA[l * ls + k] = c2r_pre(bufX + l * ls, k, M, twL);
-    }
+    W.each(nl, M, [&](int l, int k) { bufA[l * ls + k] = c2r_pre(bufX + l * ls, k, M, twL); });
     __syncthreads();
     cplx<float> *Z = block_fft(bufA, bufB, plan, nl, ls, 1, +1, false);
     cplx<float> *G = (Z == bufA) ? bufB : bufA;
     const float bg = a.bgLevel[2 * b];
     // one thread per complex point = two data columns
-    for (int idx = threadIdx.x; idx < nl * M; idx += blockDim.x) {
-      const int l = byM.div(idx), k = idx - l * M;
+    W.each(nl, M, [&](int l, int k) {
       const int row = row0 + l;
       const cplx<float> zz = Z[l * ls + k];
       float gv[2] = {0.f, 0.f};
@@ -1076,15 +1102,14 @@ __global__ void __launch_bounds__(1024) k_fast_stat_rows(FastArgs a, FastGeom g,
         gv[e] = gz;
       }
       G[l * ls + k] = {gv[0], gv[1]};
-    }
+    });
     __syncthreads();
     if (wantGrad) {
       cplx<float> *other = (G == bufA) ? bufB : bufA;
       cplx<float> *R = block_fft(G, other, plan, nl, ls, 1, -1, false);
-      for (int idx = threadIdx.x; idx < nl * (M + 1); idx += blockDim.x) {
-        const int l = byM1.div(idx), k = idx - l * (M + 1);
+      W.each(nl, M + 1, [&](int l, int k) {
         spec[(long)(row0 + l) * g.specPitch + k] = r2c_post(R + l * ls, k, M, twL);
-      }
+      });
     }
   }
   pdl_trigger();
@@ -1103,46 +1128,58 @@ __global__ void __launch_bounds__(1024) k_fast_stat_rows(FastArgs a, FastGeom g,
 // acc[0..1+NP] += r~ * dm/dtheta over the CTA's window pixels for component cc
 // (X0, Y0, then its function parameters); subsampled pixels from the table.
 template <int TY, bool REG, bool BOX>
-__device__ __forceinline__ void grad_pixels(const CompF32 cc, const WinDesc &w, const float *rt, int ls, int row0,
-                                            int npix, const FastDiv &byCols, const float *tab, int side, int bc0,
-                                            int br0, float *acc) {
+__device__ __forceinline__ void grad_pixels(const CompF32 cc, const WinDesc &w, const LineWalk &W, const float *rt,
+                                            int ls, int row0, int nl, const float *tab, int side, int bc0, int br0,
+                                            float *acc) {
   constexpr int NP = n_fparams<TY>();
   float o[7];
-  for (int idx = threadIdx.x; idx < npix; idx += blockDim.x) {
-    const int l = byCols.div(idx), col = idx - l * w.cols;
+  GradSums<TY> sums;
+  for (int l = W.l0; l < nl; l += W.dl) {
     const int row = row0 + l;
-    const float r = rt[2 * l * ls + col];
-    float dx, dy;
-    win_offsets_t<REG>(w, cc, row, col, dx, dy);
-    if constexpr (TY == F_TILTEDSKY) {
-      if (r == 0.f) continue;
-      plane_grad32(cc, dx, dy, r, o);
-    } else {
-      const Geo g = geo32(cc, dx, dy);
-      if (BOX && subsampling_t<TY>() && g.r2 < 100.f) {
-        const int ns = n_subsamples32(cc, fast_sqrt(g.r2));
-        if (ns > 1) {
-          const int br = row - br0, bc = col - bc0;
-          if (br >= 0 && br < side && bc >= 0 && bc < side) {
-            const float *t = tab + ((long)br * side + bc) * 8 + 1;
+    const float *rl = rt + 2 * l * ls;
+    float dxf, dyf;
+    win_offsets_t<false>(w, cc, row, 0, dxf, dyf);
+    float xi = (float)(W.k0 + w.xOrig - cc.x0i);
+    const float step = (float)W.dk;
+    for (int col = W.k0; col < w.cols; col += W.dk, xi += step) {
+      const float r = rl[col];
+      float dx = xi - cc.x0r, dy = dyf;
+      if constexpr (REG) win_offsets_t<REG>(w, cc, row, col, dx, dy);
+      if constexpr (TY == F_TILTEDSKY) {
+        if (r == 0.f) continue;
+        plane_grad32(cc, dx, dy, r, o);
 #pragma unroll
-            for (int q = 0; q < 2 + NP; q++) acc[q] += r * t[q];
-          } else {
-            // outside the precomputed box (not reached for radius < 10): direct average
-            const float d = 1.f / ns;
-            for (int t = 0; t < ns * ns; t++) {
-              const Geo gs = geo32(cc, dx - 0.5f + (t / ns + 0.5f) * d, dy - 0.5f + (t % ns + 0.5f) * d);
-              radial_grad_t<TY>(cc, gs, r * d * d, o);
+        for (int q = 0; q < 2 + NP; q++) acc[q] += o[q];
+      } else {
+        const Geo g = geo32(cc, dx, dy);
+        if (BOX && subsampling_t<TY>() && g.r2 < 100.f) {
+          const int ns = n_subsamples32(cc, fast_sqrt(g.r2));
+          if (ns > 1) {
+            const int br = row - br0, bc = col - bc0;
+            if (br >= 0 && br < side && bc >= 0 && bc < side) {
+              const float *t = tab + ((long)br * side + bc) * 8 + 1;
 #pragma unroll
-              for (int q = 0; q < 2 + NP; q++) acc[q] += o[q];
+              for (int q = 0; q < 2 + NP; q++) acc[q] += r * t[q];
+            } else {
+              // outside the precomputed box (not reached for radius < 10): direct average
+              const float d = 1.f / ns;
+              for (int t = 0; t < ns * ns; t++) {
+                const Geo gs = geo32(cc, dx - 0.5f + (t / ns + 0.5f) * d, dy - 0.5f + (t % ns + 0.5f) * d);
+                radial_grad_t<TY>(cc, gs, r * d * d, o);
+#pragma unroll
+                for (int q = 0; q < 2 + NP; q++) acc[q] += o[q];
+              }
             }
+            continue;
           }
-          continue;
         }
+        if (r == 0.f) continue;
+        sums.add(cc, g, r);
       }
-      if (r == 0.f) continue;
-      radial_grad_t<TY>(cc, g, r, o);
     }
+  }
+  if constexpr (TY != F_TILTEDSKY) {
+    sums.fold(cc, o);
 #pragma unroll
     for (int q = 0; q < 2 + NP; q++) acc[q] += o[q];
   }
@@ -1150,14 +1187,14 @@ __device__ __forceinline__ void grad_pixels(const CompF32 cc, const WinDesc &w, 
 
 template <int TY>
 __device__ __forceinline__ void grad_pixels_rt(bool reg, bool box, const CompF32 &cc, const WinDesc &w,
-                                               const float *rt, int ls, int row0, int npix, const FastDiv &byCols,
+                                               const LineWalk &W, const float *rt, int ls, int row0, int nl,
                                                const float *tab, int side, int bc0, int br0, float *acc) {
   if (reg) {
-    if (box) grad_pixels<TY, true, true>(cc, w, rt, ls, row0, npix, byCols, tab, side, bc0, br0, acc);
-    else grad_pixels<TY, true, false>(cc, w, rt, ls, row0, npix, byCols, tab, side, bc0, br0, acc);
+    if (box) grad_pixels<TY, true, true>(cc, w, W, rt, ls, row0, nl, tab, side, bc0, br0, acc);
+    else grad_pixels<TY, true, false>(cc, w, W, rt, ls, row0, nl, tab, side, bc0, br0, acc);
   } else {
-    if (box) grad_pixels<TY, false, true>(cc, w, rt, ls, row0, npix, byCols, tab, side, bc0, br0, acc);
-    else grad_pixels<TY, false, false>(cc, w, rt, ls, row0, npix, byCols, tab, side, bc0, br0, acc);
+    if (box) grad_pixels<TY, false, true>(cc, w, W, rt, ls, row0, nl, tab, side, bc0, br0, acc);
+    else grad_pixels<TY, false, false>(cc, w, W, rt, ls, row0, nl, tab, side, bc0, br0, acc);
   }
 }
 
@@ -1188,27 +1225,19 @@ __global__ void __launch_bounds__(1024) k_fast_grad_rows(FastArgs a, WinDesc w, 
   const int row0 = blockIdx.x * rpb;
   const int nl = min(rpb, w.rows - row0);
   const cplx<float> *spec = w.spec + (long)b * w.specBatch;
-  const FastDiv byM(M), byM1(M + 1), byCols(w.cols);
-  for (int idx = threadIdx.x; idx < max(nl, 0) * (M + 1); idx += blockDim.x) {
-    const int l = byM1.div(idx), k = idx - l * (M + 1);
-    bufX[l * ls + k] = spec[(long)(row0 + l) * w.specPitch + k];
-  }
+  const LineWalk W(max(nl, 1));
+  W.each(nl, M + 1, [&](int l, int k) { bufX[l * ls + k] = spec[(long)(row0 + l) * w.specPitch + k]; });
   __syncthreads();
   if (nl > 0) {
-    for (int idx = threadIdx.x; idx < nl * M; idx += blockDim.x) {
-      const int l = byM.div(idx), k = idx - l * M;
-      bufA[l * ls + k] = c2r_pre(bufX + l * ls, k, M, twL);
-    }
+    W.each(nl, M, [&](int l, int k) { bufA[l * ls + k] = c2r_pre(bufX + l * ls, k, M, twL); });
     __syncthreads();
     cplx<float> *Z = block_fft(bufA, bufB, plan, nl, ls, 1, +1, false);
     const float *rt = reinterpret_cast<const float *>(Z);  // r~ of (l, col) at rt[2*(l*ls) + col]
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int npix = nl * w.cols;
     if (w.losRt)
-      for (int idx = threadIdx.x; idx < npix; idx += blockDim.x) {
-        const int l = byCols.div(idx), col = idx - l * w.cols;
+      W.each(nl, w.cols, [&](int l, int col) {
         w.losRt[((long)b * w.rows + row0 + l) * w.cols + col] = rt[2 * l * ls + col];
-      }
+      });
     for (int c = 0; c < nC; c++) {
       const CompF32 cc = sc[c];
       if (!in_rows(cc.type)) continue;
@@ -1218,13 +1247,13 @@ __global__ void __launch_bounds__(1024) k_fast_grad_rows(FastArgs a, WinDesc w, 
       const bool box = rows_meet_box(cc, row0, nl, br0, side);
       float acc[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       switch (cc.type) {
-        case F_SERSIC: grad_pixels_rt<F_SERSIC>(w.isRegion, box, cc, w, rt, ls, row0, npix, byCols, tab, side, bc0, br0, acc); break;
-        case F_EXP: grad_pixels_rt<F_EXP>(w.isRegion, box, cc, w, rt, ls, row0, npix, byCols, tab, side, bc0, br0, acc); break;
-        case F_GRING: grad_pixels_rt<F_GRING>(w.isRegion, box, cc, w, rt, ls, row0, npix, byCols, tab, side, bc0, br0, acc); break;
-        case F_MOFFAT: grad_pixels_rt<F_MOFFAT>(w.isRegion, box, cc, w, rt, ls, row0, npix, byCols, tab, side, bc0, br0, acc); break;
-        case F_GAUSS: grad_pixels_rt<F_GAUSS>(w.isRegion, box, cc, w, rt, ls, row0, npix, byCols, tab, side, bc0, br0, acc); break;
+        case F_SERSIC: grad_pixels_rt<F_SERSIC>(w.isRegion, box, cc, w, W, rt, ls, row0, nl, tab, side, bc0, br0, acc); break;
+        case F_EXP: grad_pixels_rt<F_EXP>(w.isRegion, box, cc, w, W, rt, ls, row0, nl, tab, side, bc0, br0, acc); break;
+        case F_GRING: grad_pixels_rt<F_GRING>(w.isRegion, box, cc, w, W, rt, ls, row0, nl, tab, side, bc0, br0, acc); break;
+        case F_MOFFAT: grad_pixels_rt<F_MOFFAT>(w.isRegion, box, cc, w, W, rt, ls, row0, nl, tab, side, bc0, br0, acc); break;
+        case F_GAUSS: grad_pixels_rt<F_GAUSS>(w.isRegion, box, cc, w, W, rt, ls, row0, nl, tab, side, bc0, br0, acc); break;
         case F_TILTEDSKY:
-          grad_pixels_rt<F_TILTEDSKY>(w.isRegion, box, cc, w, rt, ls, row0, npix, byCols, tab, side, bc0, br0, acc);
+          grad_pixels_rt<F_TILTEDSKY>(w.isRegion, box, cc, w, W, rt, ls, row0, nl, tab, side, bc0, br0, acc);
           break;
         default: break;
       }

@@ -1767,7 +1767,12 @@ struct imfit_model_s {
     // launch shapes for the current plan: row shapes with the automatic
     // column shape, then column shapes with the best row shape
     auto tuneShapes = [&](FastTune &bestT, float &bestMs) -> cudaError_t {
-      const int rowShapes[][2] = {{1, 128}, {1, 256}, {2, 256}, {3, 256}, {4, 256}, {2, 512}, {4, 512}};
+      // (one warp a line, {3, 96} and {4, 128}, is for full GPUs: an FFT pass
+      // over a line has about n / 8 items, so more threads idle at its
+      // barriers, and small CTAs overlap one another's phases.  256 vectors of
+      // 512 x 512, {4, 256} against {3, 96}: eval 512 / 414 us, statistic
+      // 780 / 729, gradient 934 / 810)
+      const int rowShapes[][2] = {{1, 128}, {1, 256}, {2, 256}, {3, 96}, {3, 256}, {4, 128}, {4, 256}, {2, 512}, {4, 512}};
       bestT = FastTune{};
       bestMs = 1e30f;
       for (auto &rs : rowShapes) {
