@@ -68,27 +68,22 @@ __device__ __forceinline__ bool subsampling_type(int t) {
   return t == F_SERSIC || t == F_EXP || t == F_MOFFAT || t == F_GAUSS;
 }
 
-// How the threads of a CTA share nl lines: where the warps divide evenly among
-// the lines, each warp keeps to one line (first line l0, step dl) and strides
-// over its points (first k0, step dk); else all warps take the lines one after
-// the other.  A warp's line index and everything derived from it are then
-// loop constants, and a step along the line costs one addition, where a flat
-// index costs a division (four instructions, two of them on the SFU) and two
-// integer-to-float conversions a point.  256 vectors of a 512 x 512 image,
-// three components, same launch shape (4 lines, 256 threads): eval 531 to 512
-// us; gradient, with GradSums, 1057 to 934 us.
+// How the threads of a CTA share nl lines: each warp keeps to one line (first
+// line l0, step dl) with as many other warps as divide evenly (wpl), and
+// strides over its points (first k0, step dk).  A warp's line index and
+// everything derived from it are then loop constants, and a step along the
+// line costs one addition, where a flat index costs a division (four
+// instructions, two of them on the SFU) and two integer-to-float conversions a
+// point.  256 vectors of a 512 x 512 image, three components, same launch
+// shape (4 lines, 256 threads): eval 531 to 512 us; gradient, with GradSums,
+// 1057 to 934 us.
 struct LineWalk {
   int l0, dl, k0, dk;
   __device__ __forceinline__ explicit LineWalk(int nl) {
     const int nw = blockDim.x >> 5, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int wpl = FastDiv(nl).div(nw);  // warps per line
-    if (wpl < 1 || wpl * nl != nw) {
-      wpl = nw;
-      dl = 1;
-    } else {
-      dl = nl;
-    }
-    l0 = FastDiv(wpl).div(wid);
+    const int wpl = max(FastDiv(nl).div(nw), 1);  // warps per line
+    l0 = FastDiv(wpl).div(wid);                   // nl or more: nothing left for this warp
+    dl = min(nl, nw);
     k0 = (wid - l0 * wpl) * 32 + lane;
     dk = wpl * 32;
   }
@@ -622,10 +617,13 @@ __device__ __forceinline__ void eval_pixels_rt(bool reg, bool box, const CompF32
 
 __global__ void __launch_bounds__(1024) k_fast_eval_r2c(FastArgs a, WinDesc w, FFTPlan<float> plan,
                                                        const cplx<float> *__restrict__ twL, int rpb, int win) {
-  pdl_wait();
   extern __shared__ __align__(16) unsigned char smem[];
   const int b = blockIdx.y;
   const int M = plan.n, ls = M + 1;
+  const int row0 = blockIdx.x * rpb;
+  const int nl = min(rpb, w.rows - row0);
+  const LineWalk W(max(nl, 1));
+  pdl_wait();
   CompF32 *sc = reinterpret_cast<CompF32 *>(smem);
   int *boxes = reinterpret_cast<int *>(sc + kMaxComponents);
   cplx<float> *bufA = reinterpret_cast<cplx<float> *>(boxes + 2 * kMaxComponents);
@@ -637,11 +635,8 @@ __global__ void __launch_bounds__(1024) k_fast_eval_r2c(FastArgs a, WinDesc w, F
     boxes[2 * i] = o[0];
     boxes[2 * i + 1] = o[1];
   }
-  const int row0 = blockIdx.x * rpb;
-  const int nl = min(rpb, w.rows - row0);
   __syncthreads();
   if (nl <= 0) return;
-  const LineWalk W(nl);
   W.each(nl, M, [&](int l, int k) { bufA[l * ls + k] = {0.f, 0.f}; });
   const int side = win ? a.boxReg : a.boxMain;
   for (int c = 0; c < nC; c++) {
@@ -1048,18 +1043,19 @@ template <bool PS>
 __global__ void __launch_bounds__(1024) k_fast_stat_rows(FastArgs a, FastGeom g, FFTPlan<float> plan,
                                                         const cplx<float> *__restrict__ twL, int rpb, int wantGrad,
                                                         int doneTotal) {
-  pdl_wait();
   extern __shared__ __align__(16) unsigned char smem[];
   const int b = blockIdx.y;
   const int M = plan.n, ls = M + 1;
+  const int row0 = blockIdx.x * rpb;
+  const int nl = min(rpb, g.nDataRows - row0);
+  const LineWalk W(max(nl, 1));
+  pdl_wait();
   cplx<float> *bufX = reinterpret_cast<cplx<float> *>(smem);
   cplx<float> *bufA = bufX + rpb * ls;
   cplx<float> *bufB = bufA + rpb * ls;
   __shared__ float psAcc[4 * kMaxPsFast];
   if constexpr (PS)
     for (int i = threadIdx.x; i < 4 * a.nPs; i += blockDim.x) psAcc[i] = 0.f;
-  const int row0 = blockIdx.x * rpb;
-  const int nl = min(rpb, g.nDataRows - row0);
   cplx<float> *spec = reinterpret_cast<cplx<float> *>(a.spec) + (long)b * g.specBatch;
   float S = 0.f, SG = 0.f;
   if (a.dataStride) {  // image stack: this entry's data and weights
@@ -1069,7 +1065,6 @@ __global__ void __launch_bounds__(1024) k_fast_stat_rows(FastArgs a, FastGeom g,
   }
   if (a.count && a.countStride) a.count += (a.entry ? a.entry[b] : b) * a.countStride;  // batched bootstrap
   if (nl > 0) {
-    const LineWalk W(nl);
     W.each(nl, M + 1, [&](int l, int k) { bufX[l * ls + k] = spec[(long)(row0 + l) * g.specPitch + k]; });
     __syncthreads();
     W.each(nl, M, [&](int l, int k) { bufA[l * ls + k] = c2r_pre(bufX + l * ls, k, M, twL); });
@@ -1128,10 +1123,11 @@ __global__ void __launch_bounds__(1024) k_fast_stat_rows(FastArgs a, FastGeom g,
 // acc[0..1+NP] += r~ * dm/dtheta over the CTA's window pixels for component cc
 // (X0, Y0, then its function parameters); subsampled pixels from the table.
 template <int TY, bool REG, bool BOX>
-__device__ __forceinline__ void grad_pixels(const CompF32 cc, const WinDesc &w, const LineWalk &W, const float *rt,
+__device__ __forceinline__ void grad_pixels(const CompF32 &cs, const WinDesc &w, const LineWalk &W, const float *rt,
                                             int ls, int row0, int nl, const float *tab, int side, int bc0, int br0,
                                             float *acc) {
   constexpr int NP = n_fparams<TY>();
+  const CompF32 cc = cs;
   float o[7];
   GradSums<TY> sums;
   for (int l = W.l0; l < nl; l += W.dl) {
@@ -1165,9 +1161,7 @@ __device__ __forceinline__ void grad_pixels(const CompF32 cc, const WinDesc &w, 
               const float d = 1.f / ns;
               for (int t = 0; t < ns * ns; t++) {
                 const Geo gs = geo32(cc, dx - 0.5f + (t / ns + 0.5f) * d, dy - 0.5f + (t % ns + 0.5f) * d);
-                radial_grad_t<TY>(cc, gs, r * d * d, o);
-#pragma unroll
-                for (int q = 0; q < 2 + NP; q++) acc[q] += o[q];
+                sums.add(cc, gs, r * d * d);
               }
             }
             continue;
@@ -1202,10 +1196,13 @@ __global__ void __launch_bounds__(1024) k_fast_grad_rows(FastArgs a, WinDesc w, 
                                                         const cplx<float> *__restrict__ twL, int rpb,
                                                         float2 *__restrict__ gradPart, int blockBase, int win,
                                                         int doneTotal) {
-  pdl_wait();
   extern __shared__ __align__(16) unsigned char smem[];
   const int b = blockIdx.y;
   const int M = plan.n, ls = M + 1;
+  const int row0 = blockIdx.x * rpb;
+  const int nl = min(rpb, w.rows - row0);
+  const LineWalk W(max(nl, 1));
+  pdl_wait();
   CompF32 *sc = reinterpret_cast<CompF32 *>(smem);
   int *boxes = reinterpret_cast<int *>(sc + kMaxComponents);
   cplx<float> *bufX = reinterpret_cast<cplx<float> *>(boxes + 2 * kMaxComponents);
@@ -1222,10 +1219,7 @@ __global__ void __launch_bounds__(1024) k_fast_grad_rows(FastArgs a, WinDesc w, 
     boxes[2 * i + 1] = o[1];
   }
   for (int i = threadIdx.x; i < (blockDim.x >> 5) * nP; i += blockDim.x) wpart[i] = ffloat{0.f, 0.f};
-  const int row0 = blockIdx.x * rpb;
-  const int nl = min(rpb, w.rows - row0);
   const cplx<float> *spec = w.spec + (long)b * w.specBatch;
-  const LineWalk W(max(nl, 1));
   W.each(nl, M + 1, [&](int l, int k) { bufX[l * ls + k] = spec[(long)(row0 + l) * w.specPitch + k]; });
   __syncthreads();
   if (nl > 0) {
@@ -1239,7 +1233,7 @@ __global__ void __launch_bounds__(1024) k_fast_grad_rows(FastArgs a, WinDesc w, 
         w.losRt[((long)b * w.rows + row0 + l) * w.cols + col] = rt[2 * l * ls + col];
       });
     for (int c = 0; c < nC; c++) {
-      const CompF32 cc = sc[c];
+      const CompF32 &cc = sc[c];
       if (!in_rows(cc.type)) continue;
       const int side = win ? a.boxReg : a.boxMain;
       const float *tab = a.subTab + sub_base(a, b, c, win);
