@@ -26,6 +26,31 @@ template <typename T>
 __device__ __forceinline__ cplx<T> cadd(cplx<T> a, cplx<T> b) { return {a.x + b.x, a.y + b.y}; }
 template <typename T>
 __device__ __forceinline__ cplx<T> csub(cplx<T> a, cplx<T> b) { return {a.x - b.x, a.y - b.y}; }
+// FP32: both parts in one packed instruction (the same roundings).  It does not
+// add FP32 throughput but halves the issue slots, which bound the transforms:
+// two-pass columns of 256 x 289 x 576 points 324 to 291 us, row kernels 1 to
+// 2 %; packed multiply-adds inside the radix-3, 5 and 7 butterflies gained
+// nothing more (constant pairs to load).
+__device__ __forceinline__ unsigned long long pack2(cplx<float> a) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+  return r;
+}
+__device__ __forceinline__ cplx<float> unpack2(unsigned long long v) {
+  cplx<float> r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ cplx<float> cadd(cplx<float> a, cplx<float> b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a)), "l"(pack2(b)));
+  return unpack2(r);
+}
+__device__ __forceinline__ cplx<float> csub(cplx<float> a, cplx<float> b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a)), "l"(pack2(b)));
+  return unpack2(r);
+}
 // multiply by s*i (s = +1 or -1)
 template <typename T>
 __device__ __forceinline__ cplx<T> mul_si(cplx<T> a, int s) { return s > 0 ? cplx<T>{-a.y, a.x} : cplx<T>{a.y, -a.x}; }
