@@ -2024,7 +2024,10 @@ struct imfit_model_s {
     J.stat = dS;
     J.jac = jacOut;
     cudaError_t e;
-    if (useGraphs && !timing && !jacOut) {
+    // (a caller that captures the stream gets the plain launches)
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(stream, &capturing);
+    if (useGraphs && !timing && !jacOut && capturing == cudaStreamCaptureStatusNone) {
       // a Levenberg-Marquardt fit repeats the evaluation with the same
       // arguments: from the second such call on it is captured and replayed
       // (the lockstep batch, whose size changes from round to round, is not)
