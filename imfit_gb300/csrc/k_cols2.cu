@@ -15,11 +15,11 @@
 // Half the instructions per point of the multi-pass kernel (k_cols32.cu), but
 // long straight-line code at 96 registers: a CTA takes longer, and the kernel
 // wins where many share an SM.  Measured (both sides, us): 256 spectra of 576 x
-// 289 322 / 333, 11 of 1120 x 561 90 / 131, 11 of 540 x 271 18 / 31; single spectra
-// lose (1120 x 561 24 / 16, 320 x 161 12 / 9), so launch_cols32 takes this form
-// from kTwoPassColumns columns on.  What it tried and lost: the PSF columns
-// staged in shared memory (two CTAs per SM fewer: 404), more CTAs per SM with
-// spilled registers (five: 431).
+// 289 322 / 333 (291 with packed complex additions), 11 of 1120 x 561 90 / 131,
+// 11 of 540 x 271 18 / 31; single spectra lose (1120 x 561 24 / 16, 320 x 161
+// 12 / 9), so launch_cols32 takes this form from kTwoPassColumns columns on.
+// What it tried and lost: the PSF columns staged in shared memory (two CTAs per
+// SM fewer: 404), more CTAs per SM with spilled registers (five: 431).
 // Rows at or beyond nRowsIn are implicit zeros, rows from nRowsOut on are not
 // written.
 #include <algorithm>
