@@ -1773,6 +1773,7 @@ struct imfit_model_s {
       // 512 x 512, {4, 256} against {3, 96}: eval 512 / 414 us, statistic
       // 780 / 729, gradient 934 / 810)
       const int rowShapes[][2] = {{1, 128}, {1, 256}, {2, 256}, {3, 96}, {3, 256}, {4, 128}, {4, 256}, {2, 512}, {4, 512}};
+      constexpr float kBetter = 0.99f;  // a later (larger) shape has to win by more than the noise
       bestT = FastTune{};
       bestMs = 1e30f;
       for (auto &rs : rowShapes) {
@@ -1782,7 +1783,7 @@ struct imfit_model_s {
         float ms;
         cudaError_t err = measure(t, ms);
         if (err) return err;
-        if (ms < bestMs) { bestMs = ms; bestT = t; }
+        if (ms < kBetter * bestMs) { bestMs = ms; bestT = t; }
       }
       for (int cpb : {1, 2, 4, 8}) {
         for (int nt : {0, 128, 256, 512}) {
@@ -1793,7 +1794,7 @@ struct imfit_model_s {
           float ms;
           cudaError_t err = measure(t, ms);
           if (err) return err;
-          if (ms < bestMs) { bestMs = ms; bestT = t; }
+          if (ms < kBetter * bestMs) { bestMs = ms; bestT = t; }
         }
       }
       return cudaSuccess;
